@@ -239,6 +239,7 @@ struct Solver {
     bool own_stream = false;
     DevBuf A, raw, vec, act, partials, state, map;
     DevBuf tri;       // tridiagonal preconditioner planes (TriPlane), on first use
+    DevBuf sia;       // column pivots of the FP64 solvers (k_sia_factor), on first use
     DevBuf A_sav, x_sav;      // accelerated Picard's saved matrix and velocity (cismgpu_solver_save)
     DevBuf rsum;              // the reproducible sum's exponent extremes and level sums
     DevBuf rprod;             // reproducible-sum solves: the two product fields and the flag
@@ -272,6 +273,7 @@ struct Solver {
     void destroy() {
         A.release(); raw.release(); vec.release(); act.release(); partials.release(); state.release(); map.release();
         tri.release();
+        sia.release();
         A_sav.release();
         x_sav.release();
         rsum.release();
@@ -1046,37 +1048,104 @@ struct Solver {
         return CISMGPU_OK;
     }
 
-    // z = PC(r) (+ the statement MODE fuses): precond 3/4 first run their line solves
-    // (3D: of the vertically summed residual) and halo update, then k_precond finishes.
-    template <int NCC, int MODE>
-    int apply_precond(int precond, const Ptrs &p, RedCtx rc, double *du, double *dv) {
-        cudaStream_t s = stream;
-        SolveState *st = state.as<SolveState>();
-        const double *zs = nullptr;
+    // A pointwise statement group (Upd, and a pointwise preconditioner PRE) over every node.
+    template <int UPD, int PRE = P_KEEP>
+    void node(const double *dgu = nullptr, const double *dgv = nullptr) {
+        k_node<UPD, PRE><<<dim3(nblocks(g.NQ), (unsigned)g.nz), kBlock, 0, stream>>>(g, vargs(), state.as<SolveState>(),
+                                                                                    dgu, dgv);
+    }
+
+    template <int PRE, bool DOT, int NZM>
+    void col(const ColArgs &c, RedCtx rc) {
+        k_col<PRE, DOT, NZM><<<nblocks(g.NQ, DOT ? kBlock : 64), DOT ? 2 * kBlock : 128, 0, stream>>>(g, vargs(), c, rc);
+    }
+
+    // The staggered halo of one pair of planes.
+    void halo(double *u, double *v) {
+        k_halo<<<dim3(nblocks(4LL * g.NX + 4LL * (g.NY - 4)), (unsigned)g.nz), kBlock, 0, stream>>>(
+            g, u, v, state.as<SolveState>());
+    }
+
+    bool column_solves(int precond) const {
+        return is3d && (precond == CISMGPU_PRECOND_SIA || precond == CISMGPU_PRECOND_TRIDIAG_LOCAL ||
+                        precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL);
+    }
+
+    // What a preconditioner needs of the matrix, once per solve (after k_init_state: a zero pivot
+    // of the line preconditioners ends the solve with EDIVZERO).
+    int precond_setup(int precond) {
         if (precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL) {
+            TRY(tri_setup(precond));
+            // the line solution's planes: the lines write the same positions every time
+            CU(cudaMemsetAsync(tri.as<double>() + TZS_U * g.NQ, 0, 2 * g.NQ * sizeof(double), stream));
+        }
+        if (column_solves(precond)) {
+            CU(sia.ensure((size_t)4 * nvec * sizeof(double)));
+            k_sia_factor<<<dim3(nblocks(g.NQ, 128), 2), 128, 0, stream>>>(g, A.as<double>(), act.as<int32_t>(),
+                                                                          sia.as<double>());
+            CU(cudaGetLastError());
+        }
+        return CISMGPU_OK;
+    }
+
+    // The statements upd, then z = PC(r); DOT: and the sum (r,z) with rc's epilogue (setd: and
+    // d = z).  precond 3/4 first run their line solves (3D: of the vertically summed residual).
+    // One launch, except for the line preconditioners (2D: their halo update as well).
+    template <int NCC, bool DOT>
+    int precond_step(int upd, int precond, RedCtx rc, int setd = 0) {
+        const Ptrs p = ptrs();
+        SolveState *st = state.as<SolveState>();
+        const bool tri_pc = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
+        const long long bs = (long long)NCC * nvec, cd = (long long)(NCC / 2) * nvec;
+        const double *Au = A.as<double>(), *Av = Au + 3 * bs;
+        ColArgs c{};
+        c.act = act.as<int32_t>();
+        c.setd = setd;
+        if (tri_pc) {
+            if (upd == U_CG) node<U_CG>();
+            else if (upd == U_XR) node<U_XR>();
+            if (upd != U_RHALO) upd = U_NONE;
             const int global = precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
             double *T = tri.as<double>();
             const long long NQ = g.NQ;
             const unsigned lb = (tri_lines(g) + kBlock - 1) / kBlock;
-            const unsigned hb = nblocks(4LL * g.NX + 4LL * (g.NY - 4));
             if (NCC == 27) {
-                k_tri_vsum<<<nblocks(NQ), kBlock, 0, s>>>(g, p.ru, p.rv, T, st);
-                CU(cudaMemsetAsync(T + TZS_U * NQ, 0, 2 * NQ * sizeof(double), s));
-                k_tri_lines<<<lb, kBlock, 0, s>>>(g, global, T + TRS_U * NQ, T + TRS_V * NQ, T + TZS_U * NQ,
-                                                  T + TZS_V * NQ, T, st);
-                Geom g1 = g;
-                g1.nz = 1;
-                k_halo<<<hb, kBlock, 0, s>>>(g1, T + TZS_U * NQ, T + TZS_V * NQ, st);
-                zs = T + TZS_U * NQ;
+                k_tri_vsum<<<nblocks(NQ), kBlock, 0, stream>>>(g, p.ru, p.rv, T, st);
+                k_tri_lines<<<lb, kBlock, 0, stream>>>(g, global, T + TRS_U * NQ, T + TRS_V * NQ, T + TZS_U * NQ,
+                                                       T + TZS_V * NQ, T, st);
+                c.zs = T + TZS_U * NQ;
             } else {
-                CU(cudaMemsetAsync(p.zu, 0, NQ * sizeof(double), s));
-                CU(cudaMemsetAsync(p.zv, 0, NQ * sizeof(double), s));
-                k_tri_lines<<<lb, kBlock, 0, s>>>(g, global, p.ru, p.rv, p.zu, p.zv, T, st);
-                k_halo<<<hb, kBlock, 0, s>>>(g, p.zu, p.zv, st);
+                CU(cudaMemsetAsync(p.zu, 0, NQ * sizeof(double), stream));
+                CU(cudaMemsetAsync(p.zv, 0, NQ * sizeof(double), stream));
+                k_tri_lines<<<lb, kBlock, 0, stream>>>(g, global, p.ru, p.rv, p.zu, p.zv, T, st);
+                halo(p.zu, p.zv);
             }
         }
-        k_precond<MODE><<<nblocks(g.NQ), kBlock, 0, s>>>(g, precond, A.as<double>(), NCC, act.as<int32_t>(), p.ru,
-                                                         p.rv, p.zu, p.zv, du, dv, rc, zs);
+        c.upd = upd;
+        if (column_solves(precond)) {
+            c.fac = sia.as<double>();
+            c.lo[0] = Au + 4 * nvec;
+            c.lo[1] = Av + 4 * nvec;
+            if (g.nz <= 16) col<P_SIA, DOT, 16>(c, rc);
+            else if (g.nz <= 32) col<P_SIA, DOT, 32>(c, rc);
+            else col<P_SIA, DOT, 0>(c, rc);
+        } else if (precond == CISMGPU_PRECOND_NONE) {
+            if (DOT) col<P_NONE, true, 0>(c, rc);
+            else if (upd == U_CG) node<U_CG, P_NONE>();
+            else if (upd == U_RHALO) node<U_RHALO, P_NONE>();
+            else node<U_NONE, P_NONE>();
+        } else if (precond == CISMGPU_PRECOND_DIAG) {
+            c.dg[0] = Au + cd;
+            c.dg[1] = Av + cd;
+            if (DOT) col<P_DIAG, true, 0>(c, rc);
+            else if (upd == U_CG) node<U_CG, P_DIAG>(c.dg[0], c.dg[1]);
+            else if (upd == U_RHALO) node<U_RHALO, P_DIAG>(c.dg[0], c.dg[1]);
+            else node<U_NONE, P_DIAG>(c.dg[0], c.dg[1]);
+        } else {  // 2D line solves (z is theirs), or no branch of the reference taken: z unchanged
+            if (DOT) col<P_KEEP, true, 0>(c, rc);
+            else if (upd == U_CG) node<U_CG>();
+            else if (upd == U_RHALO) node<U_RHALO>();
+        }
         CU(cudaGetLastError());
         return CISMGPU_OK;
     }
@@ -1156,35 +1225,34 @@ int Solver::run_standard(int precond, int ncheck, double tol, int maxiters) {
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const VecArgs v = vargs();
     const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const unsigned nb = nblocks(g.NQ);
-    const unsigned hb = nblocks(4LL * g.NX + 4LL * (g.NY - 4));
     auto rc = [&](int epi, int iter) { return RedCtx{part, st, epi, iter}; };
     const Geom gg = g;
     prof_bytes = mv_bytes(0);
 
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
-    if (precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL)
-        TRY(tri_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+    TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
+    halo(p.xu, p.xv);
     launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr,
                                               nullptr, rc(EPI_NONE, 0));
-    k_vec<OP_STD_INIT><<<nb, kBlock, 0, s>>>(gg, v, rc(EPI_L2RHS, 0));
+    node<U_STD_INIT>();
+    k_dot_bb<<<nb, kBlock, 0, s>>>(gg, p.bu, p.bv, rc(EPI_L2RHS, 0));
     CU(cudaGetLastError());
     Poller poll(*this);
+    int upd = U_NONE;  // an unchecked iteration's update runs with the next one's preconditioner
     for (int iter = 1; iter <= maxiters; ++iter) {
-        TRY((apply_precond<NCC, PRE_STD>(precond, p, rc(EPI_STD_ETA1, iter), nullptr, nullptr)));
-        k_vec<OP_STD_D><<<nb, kBlock, 0, s>>>(gg, v, rc(EPI_NONE, iter));
-        k_halo<<<hb, kBlock, 0, s>>>(gg, p.du, p.dv, st);
+        TRY((precond_step<NCC, true>(upd, precond, rc(EPI_STD_ETA1, iter))));
+        node<U_DIR>();
         TRY(timed([&] {
             launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr,
                                                    nullptr, rc(EPI_STD_ETA2, iter));
         }));
-        k_vec<OP_XR><<<nb, kBlock, 0, s>>>(gg, v, rc(EPI_NONE, iter));
+        upd = U_XR;
         if (is_check(iter, ncheck)) {
-            k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+            node<U_XR_X>();
+            upd = U_NONE;
             launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv,
                                                       rc(EPI_CHECK, iter));
             CU(cudaGetLastError());
@@ -1193,6 +1261,7 @@ int Solver::run_standard(int precond, int ncheck, double tol, int maxiters) {
             if (f) break;
         }
     }
+    if (upd == U_XR) node<U_XR>();  // maxiters reached without a check
     CU(cudaGetLastError());
     return CISMGPU_OK;
 }
@@ -1204,11 +1273,9 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const VecArgs v = vargs();
     const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const unsigned nb = nblocks(g.NQ);
-    const unsigned hb = nblocks(4LL * g.NX + 4LL * (g.NY - 4));
     auto rc = [&](int epi, int iter) { return RedCtx{part, st, epi, iter}; };
     const Geom gg = g;
     prof_bytes = mv_bytes(1);  // the fused (r,z) dot also reads r
@@ -1217,41 +1284,42 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     if (tri && NCC == 9) maxiters = 100;
 
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
-    if (tri) TRY(tri_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
+    TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     // r = d = z = q = Az = 0 (:3048-3061)
     CU(cudaMemsetAsync(p.ru, 0, (size_t)(VAZ_V - VR_U + 1) * nvec * sizeof(double), s));
-    k_vec<OP_DOT_BB><<<nb, kBlock, 0, s>>>(gg, v, rc(EPI_L2RHS, 0));
+    k_dot_bb<<<nb, kBlock, 0, s>>>(gg, p.bu, p.bv, rc(EPI_L2RHS, 0));
     // first pass (:3085-3290)
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+    halo(p.xu, p.xv);
     launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr,
                                               nullptr, rc(EPI_NONE, 1));
-    k_vec<OP_CG_INIT><<<nb, kBlock, 0, s>>>(gg, v, rc(EPI_NONE, 1));
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.ru, p.rv, st);
-    TRY((apply_precond<NCC, PRE_CG_FIRST>(precond, p, rc(EPI_CG_RHO0, 1), p.du, p.dv)));
+    node<U_CG_INIT>();
+    TRY((precond_step<NCC, true>(U_RHALO, precond, rc(EPI_CG_RHO0, 1), 1)));  // and the halo of r, d = z
     launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr,
                                            rc(EPI_CG_FIRST, 1));
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.qu, p.qv, st);
-    k_vec<OP_XR><<<nb, kBlock, 0, s>>>(gg, v, rc(EPI_NONE, 1));
+    node<U_XR_Q>();  // the halo of q, x and r
     CU(cudaGetLastError());
     Poller poll(*this);
+    int upd = U_NONE;  // an unchecked iteration's update, or the halo of r after a check, runs with
+                       // the next iteration's preconditioner
     for (int iter = 2; iter <= maxiters; ++iter) {
-        TRY((apply_precond<NCC, PRE_ONLY>(precond, p, rc(EPI_NONE, iter), nullptr, nullptr)));
+        TRY((precond_step<NCC, false>(upd, precond, rc(EPI_NONE, iter))));
         TRY(timed([&] {
             launch_mv<NCC, MV_CG_AZ>(s, gg, Ad, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru,
                                                       p.rv, rc(EPI_CG_ITER, iter));
         }));
-        k_halo<<<hb, kBlock, 0, s>>>(gg, p.Azu, p.Azv, st);
-        k_vec<OP_CG_UPD><<<nb, kBlock, 0, s>>>(gg, v, rc(EPI_NONE, iter));
+        upd = U_CG;
         if (is_check(iter, ncheck)) {
+            node<U_CG>();
             launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv,
                                                       rc(EPI_CHECK, iter));
-            k_halo<<<hb, kBlock, 0, s>>>(gg, p.ru, p.rv, st);
+            upd = U_RHALO;  // with the next preconditioner
             CU(cudaGetLastError());
             int f = poll.after_check();
             if (f < 0) return fail(CISMGPU_ECUDA, "polling the convergence flag failed");
             if (f) break;
         }
     }
+    if (upd == U_CG) node<U_CG>();  // maxiters reached without a check
     CU(cudaGetLastError());
     return CISMGPU_OK;
 }
@@ -1268,38 +1336,34 @@ int Solver::run_standard_repro(int precond, int ncheck, double tol, int maxiters
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const VecArgs v = vargs();
     const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
-    const unsigned nb = nblocks(g.NQ);
-    const unsigned hb = nblocks(4LL * g.NX + 4LL * (g.NY - 4));
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
     double S0 = 0.0;
 
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
-    if (precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL)
-        TRY(tri_setup(precond));
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+    TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
+    halo(p.xu, p.xv);
     launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
-    k_vec<OP_STD_INIT><<<nb, kBlock, 0, s>>>(gg, v, none);
+    node<U_STD_INIT>();
     CU(cudaGetLastError());
     TRY(repro_dot(p.bu, p.bu, p.bv, p.bv, &S0));
     TRY(repro_epilogue(EPI_L2RHS, 0, S0, 0.0));
     for (int iter = 1; iter <= maxiters; ++iter) {
-        TRY((apply_precond<NCC, PRE_STD>(precond, p, none, nullptr, nullptr)));
+        TRY((precond_step<NCC, false>(U_NONE, precond, none)));
         TRY(repro_dot(p.ru, p.zu, p.rv, p.zv, &S0));
         TRY(repro_epilogue(EPI_STD_ETA1, iter, S0, 0.0));
-        k_vec<OP_STD_D><<<nb, kBlock, 0, s>>>(gg, v, none);
-        k_halo<<<hb, kBlock, 0, s>>>(gg, p.du, p.dv, st);
+        node<U_DIR>();
         launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
         CU(cudaGetLastError());
         TRY(repro_dot(p.du, p.qu, p.dv, p.qv, &S0));
         TRY(repro_epilogue(EPI_STD_ETA2, iter, S0, 0.0));
-        k_vec<OP_XR><<<nb, kBlock, 0, s>>>(gg, v, none);
         int done = 0;
-        if (is_check(iter, ncheck)) {
-            k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+        if (!is_check(iter, ncheck)) {
+            node<U_XR>();
+        } else {
+            node<U_XR_X>();
             launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
             CU(cudaGetLastError());
             TRY(repro_dot(p.ru, p.ru, p.rv, p.rv, &S0));
@@ -1322,11 +1386,8 @@ int Solver::run_chrongear_repro(int precond, int ncheck, double tol, int maxiter
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const VecArgs v = vargs();
     const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
-    const unsigned nb = nblocks(g.NQ);
-    const unsigned hb = nblocks(4LL * g.NX + 4LL * (g.NY - 4));
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
     const bool tri = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
@@ -1334,43 +1395,43 @@ int Solver::run_chrongear_repro(int precond, int ncheck, double tol, int maxiter
     double S0 = 0.0, S1 = 0.0;
 
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
-    if (tri) TRY(tri_setup(precond));
+    TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     CU(cudaMemsetAsync(p.ru, 0, (size_t)(VAZ_V - VR_U + 1) * nvec * sizeof(double), s));
     TRY(repro_dot(p.bu, p.bu, p.bv, p.bv, &S0));
     TRY(repro_epilogue(EPI_L2RHS, 0, S0, 0.0));
     // first pass
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+    halo(p.xu, p.xv);
     launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
-    k_vec<OP_CG_INIT><<<nb, kBlock, 0, s>>>(gg, v, none);
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.ru, p.rv, st);
-    TRY((apply_precond<NCC, PRE_CG_FIRST>(precond, p, none, p.du, p.dv)));
+    node<U_CG_INIT>();
+    TRY((precond_step<NCC, false>(U_RHALO, precond, none)));
+    CU(cudaMemcpyAsync(p.du, p.zu, (size_t)2 * nvec * sizeof(double), cudaMemcpyDeviceToDevice, s));  // d = z
     launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
     CU(cudaGetLastError());
     TRY(repro_dot(p.ru, p.zu, p.rv, p.zv, &S0));
     TRY(repro_dot(p.du, p.qu, p.dv, p.qv, &S1));
     TRY(repro_epilogue(EPI_CG_RHO0, 1, S0, 0.0));
     TRY(repro_epilogue(EPI_CG_FIRST, 1, S1, 0.0));
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.qu, p.qv, st);
-    k_vec<OP_XR><<<nb, kBlock, 0, s>>>(gg, v, none);
+    node<U_XR_Q>();  // the halo of q, x and r
     CU(cudaGetLastError());
+    int upd = U_NONE;  // the halo of r after a check runs with the next preconditioner
     for (int iter = 2; iter <= maxiters; ++iter) {
         int done = 0;
         TRY(read_done(&done));
         if (done) break;
-        TRY((apply_precond<NCC, PRE_ONLY>(precond, p, none, nullptr, nullptr)));
+        TRY((precond_step<NCC, false>(upd, precond, none)));
+        upd = U_NONE;
         launch_mv<NCC, MV_CG_AZ>(s, gg, Ad, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru, p.rv, none);
         CU(cudaGetLastError());
         TRY(repro_dot(p.ru, p.zu, p.rv, p.zv, &S0));
         TRY(repro_dot(p.Azu, p.zu, p.Azv, p.zv, &S1));
         TRY(repro_epilogue(EPI_CG_ITER, iter, S0, S1));
-        k_halo<<<hb, kBlock, 0, s>>>(gg, p.Azu, p.Azv, st);
-        k_vec<OP_CG_UPD><<<nb, kBlock, 0, s>>>(gg, v, none);
+        node<U_CG>();
         if (is_check(iter, ncheck)) {
             launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
             CU(cudaGetLastError());
             TRY(repro_dot(p.ru, p.ru, p.rv, p.rv, &S0));
             TRY(repro_epilogue(EPI_CHECK, iter, S0, 0.0));
-            k_halo<<<hb, kBlock, 0, s>>>(gg, p.ru, p.rv, st);
+            upd = U_RHALO;  // with the next preconditioner
         }
     }
     CU(cudaGetLastError());
@@ -1388,36 +1449,32 @@ int Solver::run_standard_seq(int precond, int ncheck, double tol, int maxiters) 
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const VecArgs v = vargs();
     const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
-    const unsigned nb = nblocks(g.NQ);
-    const unsigned hb = nblocks(4LL * g.NX + 4LL * (g.NY - 4));
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
     prof_bytes = mv_bytes(0);
 
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
-    if (precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL)
-        TRY(tri_setup(precond));
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+    TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
+    halo(p.xu, p.xv);
     launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
-    k_vec<OP_STD_INIT><<<nb, kBlock, 0, s>>>(gg, v, none);
+    node<U_STD_INIT>();
     CU(cudaGetLastError());
     TRY(seq_dot(p.bu, p.bu, p.bv, p.bv, EPI_L2RHS, 0));
     Poller poll(*this);
     for (int iter = 1; iter <= maxiters; ++iter) {
-        TRY((apply_precond<NCC, PRE_STD>(precond, p, none, nullptr, nullptr)));
+        TRY((precond_step<NCC, false>(U_NONE, precond, none)));
         TRY(seq_dot(p.ru, p.zu, p.rv, p.zv, EPI_STD_ETA1, iter));
-        k_vec<OP_STD_D><<<nb, kBlock, 0, s>>>(gg, v, none);
-        k_halo<<<hb, kBlock, 0, s>>>(gg, p.du, p.dv, st);
+        node<U_DIR>();
         TRY(timed([&] {
             launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
         }));
         TRY(seq_dot(p.du, p.qu, p.dv, p.qv, EPI_STD_ETA2, iter));
-        k_vec<OP_XR><<<nb, kBlock, 0, s>>>(gg, v, none);
-        if (is_check(iter, ncheck)) {
-            k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+        if (!is_check(iter, ncheck)) {
+            node<U_XR>();
+        } else {
+            node<U_XR_X>();
             launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
             TRY(seq_dot(p.ru, p.ru, p.rv, p.rv, EPI_CHECK, iter));
             int f = poll.after_check();
@@ -1438,11 +1495,8 @@ int Solver::run_chrongear_seq(int precond, int ncheck, double tol, int maxiters)
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const VecArgs v = vargs();
     const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
-    const unsigned nb = nblocks(g.NQ);
-    const unsigned hb = nblocks(4LL * g.NX + 4LL * (g.NY - 4));
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
     prof_bytes = mv_bytes(1);
@@ -1450,33 +1504,33 @@ int Solver::run_chrongear_seq(int precond, int ncheck, double tol, int maxiters)
     if (tri && NCC == 9) maxiters = 100;
 
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
-    if (tri) TRY(tri_setup(precond));
+    TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     CU(cudaMemsetAsync(p.ru, 0, (size_t)(VAZ_V - VR_U + 1) * nvec * sizeof(double), s));
     TRY(seq_dot(p.bu, p.bu, p.bv, p.bv, EPI_L2RHS, 0));
     // first pass
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.xu, p.xv, st);
+    halo(p.xu, p.xv);
     launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
-    k_vec<OP_CG_INIT><<<nb, kBlock, 0, s>>>(gg, v, none);
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.ru, p.rv, st);
-    TRY((apply_precond<NCC, PRE_CG_FIRST>(precond, p, none, p.du, p.dv)));
+    node<U_CG_INIT>();
+    TRY((precond_step<NCC, false>(U_RHALO, precond, none)));
+    CU(cudaMemcpyAsync(p.du, p.zu, (size_t)2 * nvec * sizeof(double), cudaMemcpyDeviceToDevice, s));  // d = z
     launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
     TRY(seq_dot2(p.ru, p.zu, p.rv, p.zv, p.du, p.qu, p.dv, p.qv, EPI_CG_RHO0, EPI_CG_FIRST, 1));
-    k_halo<<<hb, kBlock, 0, s>>>(gg, p.qu, p.qv, st);
-    k_vec<OP_XR><<<nb, kBlock, 0, s>>>(gg, v, none);
+    node<U_XR_Q>();  // the halo of q, x and r
     CU(cudaGetLastError());
     Poller poll(*this);
+    int upd = U_NONE;  // the halo of r after a check runs with the next preconditioner
     for (int iter = 2; iter <= maxiters; ++iter) {
-        TRY((apply_precond<NCC, PRE_ONLY>(precond, p, none, nullptr, nullptr)));
+        TRY((precond_step<NCC, false>(upd, precond, none)));
+        upd = U_NONE;
         TRY(timed([&] {
             launch_mv<NCC, MV_CG_AZ>(s, gg, Ad, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru, p.rv, none);
         }));
         TRY(seq_dot2(p.ru, p.zu, p.rv, p.zv, p.Azu, p.zu, p.Azv, p.zv, EPI_CG_ITER, EPI_NONE, iter));
-        k_halo<<<hb, kBlock, 0, s>>>(gg, p.Azu, p.Azv, st);
-        k_vec<OP_CG_UPD><<<nb, kBlock, 0, s>>>(gg, v, none);
+        node<U_CG>();
         if (is_check(iter, ncheck)) {
             launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
             TRY(seq_dot(p.ru, p.ru, p.rv, p.rv, EPI_CHECK, iter));
-            k_halo<<<hb, kBlock, 0, s>>>(gg, p.ru, p.rv, st);
+            upd = U_RHALO;  // with the next preconditioner
             CU(cudaGetLastError());
             int f = poll.after_check();
             if (f < 0) return fail(CISMGPU_ECUDA, "polling the convergence flag failed");

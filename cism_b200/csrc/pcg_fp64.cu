@@ -77,83 +77,52 @@ __device__ void epilogue(SolveState *st, int epi, int iter, double S0, double S1
     }
 }
 
-// Called by all threads of every CTA with the thread's column partials.
+// The fixed tree over the values of a block's first 256 threads (a block of any size; the other
+// threads pass through the barriers): shuffle-down over the 32 lanes, then over the 8 warp sums.
+// Result in thread 0.  The NF trees run side by side: each is a chain of dependent additions, and
+// one after the other they would cost twice the latency.
 template <int NF>
-__device__ void reduce_and_finish(const RedCtx &rc, DD v0, DD v1) {
-    __shared__ DD sm[8];
-    __shared__ bool last;
-    DD b0 = block_tree(v0, sm);
-    DD b1 = DD{0.0, 0.0};
-    if (NF > 1) b1 = block_tree(v1, sm);
-    if (threadIdx.x == 0) {
-        rc.partials[2 * blockIdx.x + 0] = b0;
-        rc.partials[2 * blockIdx.x + 1] = b1;
-        __threadfence();
-        unsigned int t = atomicAdd(&rc.st->ticket[0], 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    DD a0{0.0, 0.0}, a1{0.0, 0.0};
-    for (unsigned int c = threadIdx.x; c < gridDim.x; c += kBlock) {
-        DD p0, p1;
-        p0.hi = __ldcg(&rc.partials[2 * c].hi);
-        p0.lo = __ldcg(&rc.partials[2 * c].lo);
-        a0 = dd_add(a0, p0);
-        if (NF > 1) {
-            p1.hi = __ldcg(&rc.partials[2 * c + 1].hi);
-            p1.lo = __ldcg(&rc.partials[2 * c + 1].lo);
-            a1 = dd_add(a1, p1);
-        }
-    }
-    DD r0 = block_tree(a0, sm);
-    DD r1 = DD{0.0, 0.0};
-    if (NF > 1) r1 = block_tree(a1, sm);
-    if (threadIdx.x == 0) {
-        rc.st->ticket[0] = 0u;
-        epilogue(rc.st, rc.epi, rc.iter, r0.hi + r0.lo, r1.hi + r1.lo);
-    }
-}
-
-// Block tree over the first 256 threads of a block of any size (the other threads pass
-// through the barriers); result in thread 0.  Same order as block_tree.
-__device__ __forceinline__ DD block_tree_first(DD v, DD *sm) {
+__device__ __forceinline__ void block_tree_first(DD &v0, DD &v1, DD (*sm)[8]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < kBlock / 32) {
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) {
-            DD o = dd_shfl_down(v, off);
-            if (lane + off < 32) v = dd_add(v, o);
+            const DD o0 = dd_shfl_down(v0, off), o1 = (NF > 1) ? dd_shfl_down(v1, off) : DD{0.0, 0.0};
+            if (lane + off < 32) {
+                v0 = dd_add(v0, o0);
+                if (NF > 1) v1 = dd_add(v1, o1);
+            }
         }
     }
     __syncthreads();  // protect 'sm' reuse across consecutive calls
-    if (warp < kBlock / 32 && lane == 0) sm[warp] = v;
+    if (warp < kBlock / 32 && lane == 0) {
+        sm[0][warp] = v0;
+        if (NF > 1) sm[1][warp] = v1;
+    }
     __syncthreads();
     if (warp == 0) {
-        DD w = (lane < 8) ? sm[lane] : DD{0.0, 0.0};
+        v0 = (lane < 8) ? sm[0][lane] : DD{0.0, 0.0};
+        if (NF > 1) v1 = (lane < 8) ? sm[1][lane] : DD{0.0, 0.0};
 #pragma unroll
         for (int off = 4; off >= 1; off >>= 1) {
-            DD o = dd_shfl_down(w, off);
-            if (lane + off < 32) w = dd_add(w, o);
+            const DD o0 = dd_shfl_down(v0, off), o1 = (NF > 1) ? dd_shfl_down(v1, off) : DD{0.0, 0.0};
+            if (lane + off < 32) {
+                v0 = dd_add(v0, o0);
+                if (NF > 1) v1 = dd_add(v1, o1);
+            }
         }
-        v = w;
     }
-    return v;
 }
 
-// reduce_and_finish for blocks of kBlock * L threads whose first kBlock threads hold the
-// values (the column sums); identical order and result to reduce_and_finish.
+// Called by all threads of every CTA; the first kBlock threads hold their columns' sums.
 template <int NF>
-__device__ void reduce_and_finish_first(const RedCtx &rc, DD v0, DD v1) {
-    __shared__ DD sm[8];
+__device__ void reduce_and_finish(const RedCtx &rc, DD v0, DD v1) {
+    __shared__ DD sm[NF][8];
     __shared__ bool last;
-    DD b0 = block_tree_first(v0, sm);
-    DD b1 = DD{0.0, 0.0};
-    if (NF > 1) b1 = block_tree_first(v1, sm);
+    block_tree_first<NF>(v0, v1, sm);
     if (threadIdx.x == 0) {
-        rc.partials[2 * blockIdx.x + 0] = b0;
-        rc.partials[2 * blockIdx.x + 1] = b1;
+        rc.partials[2 * blockIdx.x + 0] = v0;
+        rc.partials[2 * blockIdx.x + 1] = v1;
         __threadfence();
         unsigned int t = atomicAdd(&rc.st->ticket[0], 1u);
         last = (t == gridDim.x - 1);
@@ -167,19 +136,17 @@ __device__ void reduce_and_finish_first(const RedCtx &rc, DD v0, DD v1) {
             DD p0, p1;
             p0.hi = __ldcg(&rc.partials[2 * c].hi);
             p0.lo = __ldcg(&rc.partials[2 * c].lo);
-            a0 = dd_add(a0, p0);
             if (NF > 1) {
                 p1.hi = __ldcg(&rc.partials[2 * c + 1].hi);
                 p1.lo = __ldcg(&rc.partials[2 * c + 1].lo);
-                a1 = dd_add(a1, p1);
             }
+            a0 = dd_add(a0, p0);
+            if (NF > 1) a1 = dd_add(a1, p1);
         }
-    DD r0 = block_tree_first(a0, sm);
-    DD r1 = DD{0.0, 0.0};
-    if (NF > 1) r1 = block_tree_first(a1, sm);
+    block_tree_first<NF>(a0, a1, sm);
     if (threadIdx.x == 0) {
         rc.st->ticket[0] = 0u;
-        epilogue(rc.st, rc.epi, rc.iter, r0.hi + r0.lo, r1.hi + r1.lo);
+        epilogue(rc.st, rc.epi, rc.iter, a0.hi + a0.lo, a1.hi + a1.lo);
     }
 }
 
@@ -306,8 +273,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_mv_nodes(Geom g, const double *__
         }
     }
     if (FUSED) {
-        if (MODE == MV_CG_AZ) reduce_and_finish_first<2>(rc, s0, s1);
-        else reduce_and_finish_first<1>(rc, s0, s1);
+        if (MODE == MV_CG_AZ) reduce_and_finish<2>(rc, s0, s1);
+        else reduce_and_finish<1>(rc, s0, s1);
     }
     if (NC == 27 && MODE != MV_PLAIN) {
         // the last of the gridDim.y level blocks of column block blockIdx.x to finish adds the
@@ -333,8 +300,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_mv_nodes(Geom g, const double *__
             col_of(g, q, i, j);
             if (owned(g, i, j)) col_dots<MODE>(g, q, xu, xv, yu, yv, ru, rv, d0, d1);
         }
-        if (MODE == MV_CG_AZ) reduce_and_finish_first<2>(rc, d0, d1);
-        else reduce_and_finish_first<1>(rc, d0, d1);
+        if (MODE == MV_CG_AZ) reduce_and_finish<2>(rc, d0, d1);
+        else reduce_and_finish<1>(rc, d0, d1);
     }
 }
 
@@ -348,100 +315,449 @@ inline void launch_mv(cudaStream_t s, const Geom &g, const double *A, const int3
 }
 
 // ---------------------------------------------------------------------------
-// preconditioner apply over the whole array (halo included)
+// vector statements and preconditioners over the whole array (halo included)
 // ---------------------------------------------------------------------------
-// tridiag_solver (:5870-5922) on one column of the SIA matrix (easy_sia_solver :5777-5866).
-// M(-1), M(0), M(+1) are the A planes of offsets (0,0,-1), (0,0,0), (0,0,+1).
-constexpr int kMaxNz = 64;
+// The statements between two matvecs are pointwise in a node or in a column, so they share
+// launches: an iteration is bound by HBM/L2 traffic on large grids and by its launches and memory
+// round trips on small ones.  The staggered halo (k_halo) of the vectors they read or write is
+// taken at the same time: a halo position reads its source (halo_src), or the source's thread
+// writes its images (put_haloed).  Both give the values the reference's separate update leaves.
+// With one launch per statement group and one thread per column walking its levels, an iteration
+// of the 201x201x11 ice stream spent 90 us of 190 here, and its solve took 5.42 ms against 3.88 ms
+// now (SIA); the 31x31x11 dome 2.16 against 1.08 ms, SSA 401x401 (diagonal) 161 against 113 ms.
 
-__device__ void sia_column(const Geom &g, const double *__restrict__ Mlo, const double *__restrict__ Mdi,
-                           const double *__restrict__ Mup, const double *__restrict__ r, double *__restrict__ z,
-                           long long q) {
-    const int nz = g.nz;
-    const long long NQ = g.NQ;
-    double gam[kMaxNz];
-    double sol[kMaxNz];
-    // top layer: sbdiag = 0, diag = M(0), spdiag = M(+1); bottom layer: spdiag = 0
-    double beta = Mdi[q];
-    sol[0] = r[q] / beta;
-    for (int k = 1; k < nz; ++k) {
-        const double sp_prev = Mup[(long long)(k - 1) * NQ + q];  // spdiag(k-1), k-1 <= nz-1
-        const double sb = Mlo[(long long)k * NQ + q];
-        const double dg = Mdi[(long long)k * NQ + q];
-        gam[k] = sp_prev / beta;
-        beta = __dsub_rn(dg, __dmul_rn(sb, gam[k]));
-        sol[k] = __dsub_rn(r[(long long)k * NQ + q], __dmul_rn(sb, sol[k - 1])) / beta;
-    }
-    for (int k = nz - 2; k >= 0; --k) sol[k] = __dsub_rn(sol[k], __dmul_rn(gam[k + 1], sol[k + 1]));
-    for (int k = 0; k < nz; ++k) z[(long long)k * NQ + q] = sol[k];
+// Positions of the staggered halo that hold zero (outflow, no_ice).
+__device__ __forceinline__ bool zero_pos(const Geom &g, int i, int j) {
+    if (g.outflow) return i == 0 || i == g.NX - 1 || j == 0 || j == g.NY - 1;
+    if (g.no_ice) return i <= 1 || i >= g.NX - 2 || j <= 1 || j >= g.NY - 2;
+    return false;
 }
 
-enum PreMode { PRE_ONLY = 0, PRE_STD, PRE_CG_FIRST };
+// Source coordinate of a periodic halo coordinate (identity elsewhere).
+__device__ __forceinline__ int pmap(int i, int N) {
+    if (i == 0) return N - 3;
+    if (i == 1) return N - 2;
+    if (i == N - 1) return 2;
+    return i;
+}
 
-// z = PC(r) over the whole array, then optionally:
-//   PRE_STD      : S0 = (r,z)                      [:1320-1326]
-//   PRE_CG_FIRST : S0 = (r,z) kept for the first-pass epilogue; d = z   [:3215-3223]
-// kind: 0 none (z = r), 1 diag, 2 sia (3D only), 3/4 tridiagonal: in 2D z was written by
-// k_tri_lines and the halo update, in 3D the SIA columns plus the summed line solution zs
-// ([2][NQ], u then v) on every level; anything else: z unchanged.
-template <int MODE>
-__global__ void __launch_bounds__(kBlock) k_precond(Geom g, int kind, const double *__restrict__ A,
-                                                    int NC, const int32_t *__restrict__ act,
-                                                    const double *__restrict__ ru, const double *__restrict__ rv,
-                                                    double *__restrict__ zu, double *__restrict__ zv,
-                                                    double *__restrict__ du, double *__restrict__ dv,
-                                                    RedCtx rc, const double *__restrict__ zs = nullptr) {
+__device__ __forceinline__ bool periodic_halo(const Geom &g, int i, int j) {
+    return g.periodic && (i <= 1 || i == g.NX - 1 || j <= 1 || j == g.NY - 1);
+}
+
+// Column whose value (i, j) holds after the staggered halo update; -1: it holds zero.
+__device__ __forceinline__ long long halo_src(const Geom &g, int i, int j, long long q) {
+    if (zero_pos(g, i, j)) return -1;
+    if (periodic_halo(g, i, j)) return (long long)pmap(j, g.NY) * g.NX + pmap(i, g.NX);
+    return q;
+}
+
+// a(i, j) = v followed by the staggered halo update of a, by the thread of (i, j) alone: a zero
+// position stores zero, a periodic halo position nothing, any other its value and its images.
+__device__ __forceinline__ void put_haloed(const Geom &g, int i, int j, double *__restrict__ a, double v) {
+    const int NX = g.NX, NY = g.NY;
+    const long long q = (long long)j * NX + i;
+    if (zero_pos(g, i, j)) {
+        a[q] = 0.0;
+        return;
+    }
+    if (!g.periodic) {
+        a[q] = v;
+        return;
+    }
+    if (periodic_halo(g, i, j)) return;
+    a[q] = v;
+    if (i != 2 && i < NX - 3 && j != 2 && j < NY - 3) return;  // no images
+    for (int b = 0; b < 4; ++b) {
+        const int jj = (b == 0) ? j : (b == 1 ? 0 : (b == 2 ? 1 : NY - 1));
+        if (b > 0 && pmap(jj, NY) != j) continue;
+        for (int c = 0; c < 4; ++c) {
+            const int ii = (c == 0) ? i : (c == 1 ? 0 : (c == 2 ? 1 : NX - 1));
+            if (c > 0 && pmap(ii, NX) != i) continue;
+            if ((b > 0 || c > 0) && !zero_pos(g, ii, jj)) a[(long long)jj * NX + ii] = v;
+        }
+    }
+}
+
+// The statements before the preconditioner (or alone).
+enum Upd {
+    U_NONE = 0,
+    U_RHALO,      // halo of r                                            [:1478-1480, :3118-3121]
+    U_XR,         // x = x + alpha*d; r = r - alpha*q                     [:1399-1403]
+    U_XR_X,       // U_XR, then the halo of x                             [:1399-1403, :1440-1450]
+    U_XR_Q,       // the halo of q, then U_XR                             [:3268-3276]
+    U_CG,         // the halo of Az, then d = z + beta*d; q = Az + beta*q; x += alpha*d; r -= alpha*q [:3444-3459]
+    U_DIR,        // d = z + beta*d, then the halo of d                   [:1340-1350]
+    U_STD_INIT,   // r = b - z; d = 0; z = 0                              [:1190-1206]
+    U_CG_INIT,    // r = b - z                                            [:3115-3116]
+};
+
+// What follows in the same thread: nothing, z = r, or z = r / diagonal.  The column solves are
+// in k_col.
+enum Pre { P_KEEP = 0, P_NONE, P_DIAG, P_SIA };
+
+struct VecArgs {
+    const double *bu, *bv;
+    double *xu, *xv, *ru, *rv, *du, *dv, *qu, *qv, *zu, *zv;
+    const double *Azu, *Azv;
+};
+
+// One thread per node (column, level = blockIdx.y): every load of a statement group is issued at
+// once and nz * NQ/256 CTAs stream the planes (a thread per column took one round trip per level:
+// the update alone 41 us on 201x201x11, 1.9 TB/s).
+template <int UPD, int PRE>
+__global__ void __launch_bounds__(kBlock) k_node(Geom g, VecArgs v, const SolveState *st,
+                                                 const double *__restrict__ dgu, const double *__restrict__ dgv) {
+    if (st->done) return;
+    const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
+    if (q >= g.NQ) return;
+    const double alpha = st->alpha, beta = st->beta;
+    const long long kq = (long long)blockIdx.y * g.NQ, e = kq + q;
+    int i, j;
+    col_of(g, q, i, j);
+    double r1 = 0.0, r2 = 0.0;
+    if (UPD == U_STD_INIT) {
+        r1 = __dsub_rn(v.bu[e], v.zu[e]);
+        r2 = __dsub_rn(v.bv[e], v.zv[e]);
+        v.ru[e] = r1; v.rv[e] = r2;
+        v.du[e] = 0.0; v.dv[e] = 0.0;
+        v.zu[e] = 0.0; v.zv[e] = 0.0;
+        return;
+    }
+    if (UPD == U_CG_INIT) {
+        v.ru[e] = __dsub_rn(v.bu[e], v.zu[e]);
+        v.rv[e] = __dsub_rn(v.bv[e], v.zv[e]);
+        return;
+    }
+    if (UPD == U_DIR) {
+        put_haloed(g, i, j, v.du + kq, __dadd_rn(v.zu[e], __dmul_rn(beta, v.du[e])));
+        put_haloed(g, i, j, v.dv + kq, __dadd_rn(v.zv[e], __dmul_rn(beta, v.dv[e])));
+        return;
+    }
+    const double a1 = (PRE == P_DIAG) ? dgu[e] : 1.0, a2 = (PRE == P_DIAG) ? dgv[e] : 1.0;
+    const long long s = (UPD == U_RHALO || UPD == U_XR_Q || UPD == U_CG) ? halo_src(g, i, j, q) : q;
+    if (UPD == U_NONE) {
+        r1 = v.ru[e];
+        r2 = v.rv[e];
+    } else if (UPD == U_RHALO) {
+        r1 = s >= 0 ? v.ru[kq + s] : 0.0;
+        r2 = s >= 0 ? v.rv[kq + s] : 0.0;
+        if (s != q) { v.ru[e] = r1; v.rv[e] = r2; }
+    } else if (UPD == U_CG) {
+        const double d1 = __dadd_rn(v.zu[e], __dmul_rn(beta, v.du[e]));
+        const double d2 = __dadd_rn(v.zv[e], __dmul_rn(beta, v.dv[e]));
+        const double q1 = __dadd_rn(s >= 0 ? v.Azu[kq + s] : 0.0, __dmul_rn(beta, v.qu[e]));
+        const double q2 = __dadd_rn(s >= 0 ? v.Azv[kq + s] : 0.0, __dmul_rn(beta, v.qv[e]));
+        const double x1 = __dadd_rn(v.xu[e], __dmul_rn(alpha, d1));
+        const double x2 = __dadd_rn(v.xv[e], __dmul_rn(alpha, d2));
+        r1 = __dsub_rn(v.ru[e], __dmul_rn(alpha, q1));
+        r2 = __dsub_rn(v.rv[e], __dmul_rn(alpha, q2));
+        v.du[e] = d1; v.dv[e] = d2;
+        v.qu[e] = q1; v.qv[e] = q2;
+        v.xu[e] = x1; v.xv[e] = x2;
+        v.ru[e] = r1; v.rv[e] = r2;
+    } else {  // U_XR, U_XR_X, U_XR_Q
+        const double q1 = s >= 0 ? v.qu[kq + s] : 0.0, q2 = s >= 0 ? v.qv[kq + s] : 0.0;
+        const double x1 = __dadd_rn(v.xu[e], __dmul_rn(alpha, v.du[e]));
+        const double x2 = __dadd_rn(v.xv[e], __dmul_rn(alpha, v.dv[e]));
+        r1 = __dsub_rn(v.ru[e], __dmul_rn(alpha, q1));
+        r2 = __dsub_rn(v.rv[e], __dmul_rn(alpha, q2));
+        if (UPD == U_XR_Q && s != q) { v.qu[e] = q1; v.qv[e] = q2; }
+        if (UPD == U_XR_X) {
+            put_haloed(g, i, j, v.xu + kq, x1);
+            put_haloed(g, i, j, v.xv + kq, x2);
+        } else {
+            v.xu[e] = x1; v.xv[e] = x2;
+        }
+        v.ru[e] = r1; v.rv[e] = r2;
+    }
+    if (PRE == P_NONE) {
+        v.zu[e] = r1; v.zv[e] = r2;
+    } else if (PRE == P_DIAG) {  // :1238-1253 (3D), :467-480 (2D)
+        v.zu[e] = (a1 != 0.0) ? r1 / a1 : 0.0;
+        v.zv[e] = (a2 != 0.0) ? r2 / a2 : 0.0;
+    }
+}
+
+constexpr int kMaxNz = 64;
+
+// The pivots of tridiag_solver (:5870-5922) on the columns of the SIA matrix (easy_sia_solver
+// :5777-5866): beta_k and gamma_k = spdiag_{k-1} / beta_{k-1} depend on the matrix alone, so a
+// solve takes them once, with the operations of the reference's recurrence, and its column solves
+// keep one division per level instead of two.  fac: [u, v][beta, gamma][nz][NQ]; one thread per
+// active column and component, loads of kColChunk levels at a time.
+constexpr int kColChunk = 4;
+__global__ void k_sia_factor(Geom g, const double *__restrict__ A, const int32_t *__restrict__ act,
+                             double *__restrict__ fac) {
+    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= g.NQ || act[q] == 0) return;
+    const int nz = g.nz;
+    const long long NQ = g.NQ, plane = (long long)nz * NQ;
+    const double *B = A + (blockIdx.y ? 3LL : 0LL) * 27 * plane;
+    const double *Mlo = B + 4 * plane, *Mdi = B + 13 * plane, *Mup = B + 22 * plane;
+    double *fb = fac + (blockIdx.y ? 2 : 0) * plane, *fg = fb + plane;
+    double beta = Mdi[q];
+    fb[q] = beta;
+    fg[q] = 0.0;
+    for (int k0 = 1; k0 < nz; k0 += 8) {
+        double sp[8], sb[8], dg[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const long long e = (long long)(k0 + u) * NQ + q;
+            const bool in = k0 + u < nz;
+            sp[u] = in ? Mup[e - NQ] : 0.0;
+            sb[u] = in ? Mlo[e] : 0.0;
+            dg[u] = in ? Mdi[e] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (k0 + u < nz) {
+                const long long e = (long long)(k0 + u) * NQ + q;
+                const double gam = sp[u] / beta;
+                beta = __dsub_rn(dg[u], __dmul_rn(sb[u], gam));
+                fb[e] = beta;
+                fg[e] = gam;
+            }
+    }
+}
+
+struct ColArgs {
+    int upd;                    // Upd: U_NONE, U_RHALO, U_XR or U_CG
+    int setd;                   // d = z (first pass of Chronopoulos-Gear, :3215-3223)
+    const double *lo[2];        // P_SIA: the sub-diagonal planes of u and v
+    const double *fac;          // P_SIA: k_sia_factor
+    const double *dg[2];        // P_DIAG: the diagonal planes
+    const double *zs;           // line preconditioners (3D): [2][NQ] line solution, added on every level
+    const int32_t *act;
+};
+
+// One thread per (column, component): a block holds CW columns' u components, then their v
+// components.  UPD as k_node, then the preconditioner: P_SIA, the column solves of
+// tridiag_solver (:5870-5922) (+ the line solution, tridiag_solver_{local,global}_3d :4617-4655 /
+// :4876-4911), or with DOT also P_NONE, P_DIAG and P_KEEP.  Loads of kColChunk levels are issued
+// together; NZM > 0: a column of up to NZM levels stays in registers between the two sweeps, else
+// it goes through z.  DOT: S0 = (r,z) over the owned columns, per column in level order
+// (:1320-1326): the v threads hand their products to the u threads through shared memory.
+// Bound by HBM on large grids (224 bytes a node with U_CG); 64-column blocks without DOT, so that
+// 84k threads of a 201x201 grid spread over all SMs (256 are the reduction's chunk with DOT).
+template <int PRE, bool DOT, int NZM>
+__global__ void __launch_bounds__(DOT ? 2 * kBlock : 128) k_col(Geom g, VecArgs v, ColArgs c, RedCtx rc) {
+    if (rc.st->done) return;
+    constexpr int CW = DOT ? kBlock : 64;
+    constexpr int C = kColChunk;
+    __shared__ double sprod[DOT ? C : 1][DOT ? kBlock : 1];
+    const int comp = threadIdx.x >= CW ? 1 : 0, cl = threadIdx.x - comp * CW;
+    const long long q = (long long)blockIdx.x * CW + cl;
+    const int nz = g.nz;
+    const long long NQ = g.NQ, plane = (long long)nz * NQ;
+    const bool in = q < NQ;
+    const double alpha = rc.st->alpha, beta = rc.st->beta;
+    double *__restrict__ R = comp ? v.rv : v.ru;
+    double *__restrict__ Z = comp ? v.zv : v.zu;
+    double *__restrict__ D = comp ? v.dv : v.du;
+    double *__restrict__ Q = comp ? v.qv : v.qu;
+    double *__restrict__ X = comp ? v.xv : v.xu;
+    const double *__restrict__ Az = comp ? v.Azv : v.Azu;
+    const double *__restrict__ fb = c.fac + (comp ? 2 : 0) * plane, *__restrict__ fg = fb + plane;
+    const double *__restrict__ lo = comp ? c.lo[1] : c.lo[0], *__restrict__ dg = comp ? c.dg[1] : c.dg[0];
+    bool own = false, solve = false;
+    if (in) {
+        int i, j;
+        col_of(g, q, i, j);
+        own = owned(g, i, j);
+        solve = (PRE == P_SIA) && c.act[q] != 0;
+        const long long s = (c.upd == U_RHALO || c.upd == U_CG) ? halo_src(g, i, j, q) : q;
+        double y[NZM > 0 ? NZM : 1];
+        double prev = 0.0;
+        // r of C levels from k0 (the update's statements included)
+        auto chunk = [&](int k0, double (&r)[C]) {
+            if (c.upd == U_CG) {
+                double dd[C], qq[C], xx[C], zz[C], az[C];
+#pragma unroll
+                for (int u = 0; u < C; ++u) {
+                    const long long e = (long long)(k0 + u) * NQ + q;
+                    const bool on = k0 + u < nz;
+                    r[u] = on ? R[e] : 0.0;
+                    dd[u] = on ? D[e] : 0.0;
+                    qq[u] = on ? Q[e] : 0.0;
+                    xx[u] = on ? X[e] : 0.0;
+                    zz[u] = on ? Z[e] : 0.0;
+                    az[u] = (on && s >= 0) ? Az[e - q + s] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < C; ++u) {
+                    if (k0 + u >= nz) continue;
+                    const long long e = (long long)(k0 + u) * NQ + q;
+                    const double dn = __dadd_rn(zz[u], __dmul_rn(beta, dd[u]));
+                    const double qn = __dadd_rn(az[u], __dmul_rn(beta, qq[u]));
+                    r[u] = __dsub_rn(r[u], __dmul_rn(alpha, qn));
+                    D[e] = dn;
+                    Q[e] = qn;
+                    X[e] = __dadd_rn(xx[u], __dmul_rn(alpha, dn));
+                    R[e] = r[u];
+                }
+            } else if (c.upd == U_XR) {
+                double dd[C], qq[C], xx[C];
+#pragma unroll
+                for (int u = 0; u < C; ++u) {
+                    const long long e = (long long)(k0 + u) * NQ + q;
+                    const bool on = k0 + u < nz;
+                    r[u] = on ? R[e] : 0.0;
+                    dd[u] = on ? D[e] : 0.0;
+                    qq[u] = on ? Q[e] : 0.0;
+                    xx[u] = on ? X[e] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < C; ++u) {
+                    if (k0 + u >= nz) continue;
+                    const long long e = (long long)(k0 + u) * NQ + q;
+                    r[u] = __dsub_rn(r[u], __dmul_rn(alpha, qq[u]));
+                    X[e] = __dadd_rn(xx[u], __dmul_rn(alpha, dd[u]));
+                    R[e] = r[u];
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < C; ++u) {
+                    const long long e = (long long)(k0 + u) * NQ + q;
+                    r[u] = (k0 + u < nz && s >= 0) ? R[e - q + s] : 0.0;
+                }
+                if (s != q) {
+#pragma unroll
+                    for (int u = 0; u < C; ++u)
+                        if (k0 + u < nz) R[(long long)(k0 + u) * NQ + q] = r[u];
+                }
+            }
+        };
+        // forward sweep: sol_1 = r_1 / beta_1; sol_k = (r_k - sbdiag_k sol_{k-1}) / beta_k
+        auto forward = [&](int k0, double *yk) {
+            double r[C], sb[C], be[C];
+            if (PRE == P_SIA && solve) {
+#pragma unroll
+                for (int u = 0; u < C; ++u) {
+                    const long long e = (long long)(k0 + u) * NQ + q;
+                    const bool on = k0 + u < nz;
+                    sb[u] = on ? lo[e] : 0.0;
+                    be[u] = on ? fb[e] : 1.0;
+                }
+            } else if (PRE == P_DIAG) {
+#pragma unroll
+                for (int u = 0; u < C; ++u) be[u] = (k0 + u < nz) ? dg[(long long)(k0 + u) * NQ + q] : 0.0;
+            }
+            chunk(k0, r);
+#pragma unroll
+            for (int u = 0; u < C; ++u) {
+                if (k0 + u >= nz) continue;
+                const long long e = (long long)(k0 + u) * NQ + q;
+                if (PRE == P_SIA) {
+                    if (!solve) continue;
+                    prev = (k0 + u == 0) ? r[u] / be[u] : __dsub_rn(r[u], __dmul_rn(sb[u], prev)) / be[u];
+                    if (NZM > 0) yk[u] = prev;
+                    else Z[e] = prev;
+                } else if (PRE == P_NONE) {
+                    Z[e] = r[u];
+                } else if (PRE == P_DIAG) {
+                    Z[e] = (be[u] != 0.0) ? r[u] / be[u] : 0.0;
+                }
+            }
+        };
+        if (NZM > 0) {
+#pragma unroll
+            for (int k0 = 0; k0 < NZM; k0 += C)
+                if (k0 < nz) forward(k0, &y[k0]);
+        } else {
+            for (int k0 = 0; k0 < nz; k0 += C) forward(k0, y);
+        }
+        // back substitution: sol_k = sol_k - gamma_{k+1} sol_{k+1}
+        if (PRE == P_SIA && solve) {
+            if (NZM > 0) {
+#pragma unroll
+                for (int k0 = (NZM - 1) / C * C; k0 >= 0; k0 -= C) {
+                    if (k0 >= nz) continue;
+                    double ga[C];
+#pragma unroll
+                    for (int u = 0; u < C; ++u) ga[u] = (k0 + u < nz - 1) ? fg[(long long)(k0 + u + 1) * NQ + q] : 0.0;
+#pragma unroll
+                    for (int u = C - 1; u >= 0; --u) {
+                        if (k0 + u < nz - 1) y[k0 + u] = prev = __dsub_rn(y[k0 + u], __dmul_rn(ga[u], prev));
+                        if (k0 + u < nz) Z[(long long)(k0 + u) * NQ + q] = y[k0 + u];
+                    }
+                }
+            } else {
+                for (int k1 = nz - 2; k1 >= 0; k1 -= C) {
+                    double ga[C], yy[C];
+#pragma unroll
+                    for (int u = 0; u < C; ++u) {
+                        ga[u] = (k1 - u >= 0) ? fg[(long long)(k1 - u + 1) * NQ + q] : 0.0;
+                        yy[u] = (k1 - u >= 0) ? Z[(long long)(k1 - u) * NQ + q] : 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < C; ++u)
+                        if (k1 - u >= 0)
+                            Z[(long long)(k1 - u) * NQ + q] = prev = __dsub_rn(yy[u], __dmul_rn(ga[u], prev));
+                }
+            }
+        }
+        if (PRE == P_SIA && c.zs) {  // + the line solution, its halo update taken on the way
+            const long long sz = halo_src(g, i, j, q);
+            const double zl = sz >= 0 ? c.zs[(comp ? NQ : 0) + sz] : 0.0;
+            for (int k0 = 0; k0 < nz; k0 += C) {
+                double zz[C];
+#pragma unroll
+                for (int u = 0; u < C; ++u) zz[u] = (k0 + u < nz) ? Z[(long long)(k0 + u) * NQ + q] : 0.0;
+#pragma unroll
+                for (int u = 0; u < C; ++u)
+                    if (k0 + u < nz) Z[(long long)(k0 + u) * NQ + q] = __dadd_rn(zz[u], zl);
+            }
+        }
+    }
+    if (DOT) {  // the products again from r and z (this thread's own stores), C levels at a time
+        DD s0{0.0, 0.0};
+        for (int k0 = 0; k0 < nz; k0 += C) {
+            double p[C];
+#pragma unroll
+            for (int u = 0; u < C; ++u) {
+                p[u] = 0.0;
+                if (in && k0 + u < nz) {
+                    const long long e = (long long)(k0 + u) * NQ + q;
+                    const double z = Z[e];
+                    p[u] = __dmul_rn(R[e], z);
+                    if (c.setd) D[e] = z;
+                }
+                if (comp) sprod[u][cl] = p[u];
+            }
+            __syncthreads();
+            if (!comp && own) {
+#pragma unroll
+                for (int u = 0; u < C; ++u)
+                    if (k0 + u < nz) s0 = dd_add_d(s0, __dadd_rn(p[u], sprod[u][cl]));
+            }
+            __syncthreads();
+        }
+        reduce_and_finish<1>(rc, s0, s0);
+    }
+}
+
+// S0 = (b,b) over the owned columns, per column in level order (:1208-1216, :3067-3074).
+__global__ void __launch_bounds__(kBlock) k_dot_bb(Geom g, const double *__restrict__ bu, const double *__restrict__ bv,
+                                                   RedCtx rc) {
     if (rc.st->done) return;
     const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
     DD s0{0.0, 0.0};
-    if (q < g.NQ) {
-        int i, j;
-        col_of(g, q, i, j);
-        const long long plane = (long long)g.nz * g.NQ;
-        const int cdiag = (NC == 27) ? 13 : 4;
-        const double *Auu = A, *Avv = A + 3LL * NC * plane;
-        if (kind == CISMGPU_PRECOND_NONE) {
-            for (int k = 0; k < g.nz; ++k) {
-                const long long e = (long long)k * g.NQ + q;
-                zu[e] = ru[e];
-                zv[e] = rv[e];
+    int i = -1, j = -1;
+    if (q < g.NQ) col_of(g, q, i, j);
+    if (q < g.NQ && owned(g, i, j))
+        for (int k0 = 0; k0 < g.nz; k0 += 8) {
+            double t[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const long long e = (long long)(k0 + u) * g.NQ + q;
+                t[u] = (k0 + u < g.nz) ? __dadd_rn(__dmul_rn(bu[e], bu[e]), __dmul_rn(bv[e], bv[e])) : 0.0;
             }
-        } else if (kind == CISMGPU_PRECOND_DIAG) {  // :1238-1253 (3D), :467-480 (2D)
-            for (int k = 0; k < g.nz; ++k) {
-                const long long e = (long long)k * g.NQ + q;
-                const double a = Auu[(long long)cdiag * plane + e], b = Avv[(long long)cdiag * plane + e];
-                zu[e] = (a != 0.0) ? ru[e] / a : 0.0;
-                zv[e] = (b != 0.0) ? rv[e] / b : 0.0;
-            }
-        } else if (kind == CISMGPU_PRECOND_SIA && NC == 27) {  // :1255-1263
-            if (act[q] != 0) {
-                sia_column(g, Auu + 4 * plane, Auu + 13 * plane, Auu + 22 * plane, ru, zu, q);
-                sia_column(g, Avv + 4 * plane, Avv + 13 * plane, Avv + 22 * plane, rv, zv, q);
-            }
-        } else if ((kind == CISMGPU_PRECOND_TRIDIAG_LOCAL || kind == CISMGPU_PRECOND_TRIDIAG_GLOBAL) && NC == 27) {
-            // tridiag_solver_{local,global}_3d :4617-4655 / :4876-4911: SIA columns, then + zs
-            if (act[q] != 0) {
-                sia_column(g, Auu + 4 * plane, Auu + 13 * plane, Auu + 22 * plane, ru, zu, q);
-                sia_column(g, Avv + 4 * plane, Avv + 13 * plane, Avv + 22 * plane, rv, zv, q);
-            }
-            const double su = zs[q], sv = zs[g.NQ + q];
-            for (int k = 0; k < g.nz; ++k) {
-                const long long e = (long long)k * g.NQ + q;
-                zu[e] = __dadd_rn(zu[e], su);
-                zv[e] = __dadd_rn(zv[e], sv);
-            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (k0 + u < g.nz) s0 = dd_add_d(s0, t[u]);
         }
-        if (MODE == PRE_STD || MODE == PRE_CG_FIRST) {
-            const bool own = owned(g, i, j);
-            for (int k = 0; k < g.nz; ++k) {
-                const long long e = (long long)k * g.NQ + q;
-                const double z1 = zu[e], z2 = zv[e];
-                if (own) s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(ru[e], z1), __dmul_rn(rv[e], z2)));
-                if (MODE == PRE_CG_FIRST) { du[e] = z1; dv[e] = z2; }
-            }
-        }
-    }
-    if (MODE == PRE_STD || MODE == PRE_CG_FIRST) reduce_and_finish<1>(rc, s0, s0);
+    reduce_and_finish<1>(rc, s0, s0);
 }
 
 // ---------------------------------------------------------------------------
@@ -840,72 +1156,6 @@ __global__ void k_tri_lines(Geom g, int global, const double *__restrict__ bu, c
 }
 
 // ---------------------------------------------------------------------------
-// whole-array vector statements
-// ---------------------------------------------------------------------------
-enum VecOp {
-    OP_STD_INIT = 0,  // r = b - z; d = 0; z = 0; S0 = (b,b)           [:1190-1216]
-    OP_STD_D,         // d = z + beta*d                                  [:1340-1341]
-    OP_XR,            // x = x + alpha*d; r = r - alpha*q                [:1399-1403, :3272-3276]
-    OP_CG_INIT,       // r = b - z                                       [:3115-3116]
-    OP_CG_UPD,        // d = z + beta*d; q = Az + beta*q; x += alpha*d; r -= alpha*q  [:3444-3459]
-    OP_DOT_BB,        // S0 = (b,b)                                      [:3067-3074]
-};
-
-struct VecArgs {
-    const double *bu, *bv;
-    double *xu, *xv, *ru, *rv, *du, *dv, *qu, *qv, *zu, *zv;
-    const double *Azu, *Azv;
-};
-
-template <int OP>
-__global__ void __launch_bounds__(kBlock) k_vec(Geom g, VecArgs v, RedCtx rc) {
-    if (rc.st->done) return;
-    const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
-    DD s0{0.0, 0.0};
-    const double alpha = rc.st->alpha, beta = rc.st->beta;
-    if (q < g.NQ) {
-        int i, j;
-        col_of(g, q, i, j);
-        const bool own = owned(g, i, j);
-        for (int k = 0; k < g.nz; ++k) {
-            const long long e = (long long)k * g.NQ + q;
-            if (OP == OP_STD_INIT) {
-                v.ru[e] = __dsub_rn(v.bu[e], v.zu[e]);
-                v.rv[e] = __dsub_rn(v.bv[e], v.zv[e]);
-                v.du[e] = 0.0; v.dv[e] = 0.0;
-                v.zu[e] = 0.0; v.zv[e] = 0.0;
-                if (own) s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(v.bu[e], v.bu[e]), __dmul_rn(v.bv[e], v.bv[e])));
-            } else if (OP == OP_DOT_BB) {
-                if (own) s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(v.bu[e], v.bu[e]), __dmul_rn(v.bv[e], v.bv[e])));
-            } else if (OP == OP_STD_D) {
-                v.du[e] = __dadd_rn(v.zu[e], __dmul_rn(beta, v.du[e]));
-                v.dv[e] = __dadd_rn(v.zv[e], __dmul_rn(beta, v.dv[e]));
-            } else if (OP == OP_XR) {
-                v.xu[e] = __dadd_rn(v.xu[e], __dmul_rn(alpha, v.du[e]));
-                v.xv[e] = __dadd_rn(v.xv[e], __dmul_rn(alpha, v.dv[e]));
-                v.ru[e] = __dsub_rn(v.ru[e], __dmul_rn(alpha, v.qu[e]));
-                v.rv[e] = __dsub_rn(v.rv[e], __dmul_rn(alpha, v.qv[e]));
-            } else if (OP == OP_CG_INIT) {
-                v.ru[e] = __dsub_rn(v.bu[e], v.zu[e]);
-                v.rv[e] = __dsub_rn(v.bv[e], v.zv[e]);
-            } else if (OP == OP_CG_UPD) {
-                const double d1 = __dadd_rn(v.zu[e], __dmul_rn(beta, v.du[e]));
-                const double d2 = __dadd_rn(v.zv[e], __dmul_rn(beta, v.dv[e]));
-                const double q1 = __dadd_rn(v.Azu[e], __dmul_rn(beta, v.qu[e]));
-                const double q2 = __dadd_rn(v.Azv[e], __dmul_rn(beta, v.qv[e]));
-                v.du[e] = d1; v.dv[e] = d2;
-                v.qu[e] = q1; v.qv[e] = q2;
-                v.xu[e] = __dadd_rn(v.xu[e], __dmul_rn(alpha, d1));
-                v.xv[e] = __dadd_rn(v.xv[e], __dmul_rn(alpha, d2));
-                v.ru[e] = __dsub_rn(v.ru[e], __dmul_rn(alpha, q1));
-                v.rv[e] = __dsub_rn(v.rv[e], __dmul_rn(alpha, q2));
-            }
-        }
-    }
-    if (OP == OP_STD_INIT || OP == OP_DOT_BB) reduce_and_finish<1>(rc, s0, s0);
-}
-
-// ---------------------------------------------------------------------------
 // staggered halo on one rank (parallel_mpi.F90:10772-10936)
 // ---------------------------------------------------------------------------
 // Threads enumerate the ring columns: rows j in {0,1,NY-2,NY-1} (all i), then
@@ -917,13 +1167,6 @@ __global__ void __launch_bounds__(kBlock) k_vec(Geom g, VecArgs v, RedCtx rc) {
 // then zeroes i,j in {0, N-1}; no_ice zeroes i,j in {0,1,N-2,N-1}.  Levels k run over
 // blockIdx.y, blockIdx.y + gridDim.y, ... (many planes, such as the 27 nz coefficient planes of
 // a block, take a grid with several rows of blocks).
-__device__ __forceinline__ int pmap(int i, int N) {
-    if (i == 0) return N - 3;
-    if (i == 1) return N - 2;
-    if (i == N - 1) return 2;
-    return i;
-}
-
 __global__ void __launch_bounds__(kBlock) k_halo(Geom g, double *__restrict__ au, double *__restrict__ av,
                                                  const SolveState *st) {
     if (st && st->done) return;
@@ -942,11 +1185,8 @@ __global__ void __launch_bounds__(kBlock) k_halo(Geom g, double *__restrict__ au
         j = 2 + (int)(u - (long long)r * (NY - 4));
         i = (r < 2) ? r : NX - 4 + r;
     }
-    bool zero = false;
-    if (g.outflow) zero = (i == 0 || i == NX - 1 || j == 0 || j == NY - 1);
-    else if (g.no_ice) zero = (i <= 1 || i >= NX - 2 || j <= 1 || j >= NY - 2);
     const long long q = (long long)j * NX + i;
-    if (zero) {
+    if (zero_pos(g, i, j)) {
         for (int k = blockIdx.y; k < g.nz; k += gridDim.y) {
             au[(long long)k * g.NQ + q] = 0.0;
             av[(long long)k * g.NQ + q] = 0.0;
@@ -954,8 +1194,7 @@ __global__ void __launch_bounds__(kBlock) k_halo(Geom g, double *__restrict__ au
         return;
     }
     if (g.periodic) {
-        const bool halo = (i <= 1 || i == NX - 1 || j <= 1 || j == NY - 1);
-        if (!halo) return;
+        if (!periodic_halo(g, i, j)) return;
         const long long s = (long long)pmap(j, NY) * NX + pmap(i, NX);
         for (int k = blockIdx.y; k < g.nz; k += gridDim.y) {
             au[(long long)k * g.NQ + q] = au[(long long)k * g.NQ + s];

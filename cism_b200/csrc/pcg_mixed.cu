@@ -124,12 +124,6 @@ struct MCtl {
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool zero_pos(const Geom &g, int i, int j) {
-    if (g.outflow) return i == 0 || i == g.NX - 1 || j == 0 || j == g.NY - 1;
-    if (g.no_ice) return i <= 1 || i >= g.NX - 2 || j <= 1 || j >= g.NY - 2;
-    return false;
-}
-
 // Map a vertex position to the owned position whose value it holds after the
 // staggered halo update; returns -1 for positions that hold zero or lie outside
 // the array.
