@@ -1863,6 +1863,9 @@ __global__ void k_tri_to_f32(Geom g, const double *__restrict__ T, float *__rest
     }
 }
 
+// The handles' device memory (cismgpu.cu).
+void dev_free(void *p);
+
 // Device buffers of the mixed solver for one system (owned by the host Solver).
 struct MixedBufs {
     bool valid = false;
@@ -1893,7 +1896,7 @@ struct MixedBufs {
     void release() {
         for (void *p : {(void *)A32, (void *)A64i, (void *)pre, (void *)vec, (void *)recs, (void *)state, (void *)desc,
                         (void *)tiles, (void *)ctl, (void *)maps, (void *)nbrs, (void *)bc, (void *)flag, (void *)tri})
-            if (p) cudaFree(p);
+            if (p) dev_free(p);
         tri = nullptr;
         A32 = nullptr;
         A64i = nullptr;

@@ -93,6 +93,8 @@ struct cismgpu_server {
     std::thread th;                 // epoch loop
     std::thread up;                 // admissions and uploads
     cudaStream_t es = nullptr;      // epoch stream
+    cismgpu_server() { cismgpu::mem_pool().join(); }  // freed requests' memory serves the next ones
+    ~cismgpu_server() { cismgpu::mem_pool().leave(); }
     std::chrono::steady_clock::time_point t0;
     double now() const {
         return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -137,8 +139,9 @@ static int srv_admit(SrvReq &r) {
         if (owned >= kSrvResidentMin) {
             r.cls = 2;
             r.TY = ty1;
-            CU(cudaMallocHost((void **)&r.h_st, sizeof(MState)));
-            CU(cudaMallocHost((void **)&r.h_ctl, sizeof(MCtl)));
+            CU(mem_pool().take_host((void **)&r.h_st));  // one pinned block for both
+            r.h_ctl = reinterpret_cast<MCtl *>(reinterpret_cast<char *>(r.h_st) + 1024);
+            static_assert(sizeof(MState) <= 1024 && 1024 + sizeof(MCtl) <= kPoolHostBlock, "one block");
         }
     }
     TRY(mixed_prepare(sv, q.precond, r.TY));
@@ -275,8 +278,7 @@ static void srv_free(cismgpu_server *S, SrvReq &r) {
         cismgpu_solver_destroy(r.h);
         r.h = nullptr;
     }
-    if (r.h_st) cudaFreeHost(r.h_st);
-    if (r.h_ctl) cudaFreeHost(r.h_ctl);
+    if (r.h_st) mem_pool().give_host(r.h_st);
     r.h_st = nullptr;
     r.h_ctl = nullptr;
     std::lock_guard<std::mutex> lk(S->mu);
