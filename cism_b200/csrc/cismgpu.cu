@@ -301,6 +301,12 @@ static int check_device() {
 }
 
 static inline unsigned nblocks(long long n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
+// An FP64 3D solve builds the symmetric half of its matrix from this size of the full blocks and this
+// many iterations on: below, L2 keeps the planes and both products take 6.3 us (40x40x11 to 64x64x11;
+// 96x96x11 10.4 us from the planes, 9.3 from the half; 149x100x11 26.8 and 14.5; 201x201x11 59.7 and
+// 37.0), and the copy costs what three products save.
+constexpr size_t kHalfMinBytes = 64u << 20;
+constexpr int kHalfMinIters = 8;
 // rows of blocks (levels in parallel) for the halo of a matrix's 27 nz coefficient planes
 constexpr unsigned kHaloPlaneRows = 64;
 static inline bool is_check(int iter, int ncheck) { return (iter % ncheck == 0) || iter == 5; }
@@ -363,6 +369,9 @@ struct Solver {
     bool own_stream = false;
     DevBuf A, raw, vec, act, partials, state, map;
     DevBuf tri;       // tridiagonal preconditioner planes (TriPlane), on first use
+    DevBuf half;      // symmetric half of a 3D matrix (k_half3d), on first use
+    DevBuf terms;     // dot terms of a 3D matvec ([2][nz][NQ])
+    int half_state = -1;  // half holds the current matrix: 1; not exactly symmetric: 0; not tested: -1
     DevBuf sia;       // column pivots of the FP64 solvers (k_sia_factor), on first use
     DevBuf A_sav, x_sav;      // accelerated Picard's saved matrix and velocity (cismgpu_solver_save)
     DevBuf rsum;              // the reproducible sum's exponent extremes and level sums
@@ -404,6 +413,9 @@ struct Solver {
         A.release(); raw.release(); vec.release(); act.release(); partials.release(); state.release(); map.release();
         tri.release();
         sia.release();
+        half.release();
+        terms.release();
+        half_state = -1;
         A_sav.release();
         x_sav.release();
         rsum.release();
@@ -477,6 +489,7 @@ struct Solver {
         CU(partials.ensure(nbq * 2 * sizeof(DD) + nbq * sizeof(unsigned)));
         CU(cudaMemsetAsync(partials.as<DD>() + 2 * nbq, 0, nbq * sizeof(unsigned), stream));
         CU(state.ensure(sizeof(SolveState)));
+        half_state = -1;
         return CISMGPU_OK;
     }
 
@@ -503,7 +516,7 @@ struct Solver {
         CU(A.ensure(4 * blk_bytes));
         CU(raw.ensure(blk_bytes));
         cudaStream_t s = stream;
-        mixed.stale = true;  // new matrix: FP32 copy and factors must be rebuilt
+        matrix_changed();  // copies and factors must be rebuilt
         for (int b = 0; b < 4; ++b) {
             CU(h2d_copy(raw.p, blocks[b], blk_bytes, s));
             double *dst = A.as<double>() + (size_t)b * NC * nvec;
@@ -553,11 +566,11 @@ struct Solver {
         RedCtx rc1{partials.as<DD>(), st, EPI_RESID_VEC, 0};
         const unsigned nb = nblocks(g.NQ);
         if (is3d)
-            launch_mv<27, MV_PLAIN>(s, g, A.as<double>(), act.as<int32_t>(), xu, xv, p.zu, p.zv,
-                                                              nullptr, nullptr, nullptr, nullptr, rc0);
+            launch_mv<27, MV_PLAIN>(s, g, matrix(), act.as<int32_t>(), xu, xv, p.zu, p.zv, nullptr, nullptr, nullptr,
+                                    nullptr, nullptr, rc0);
         else
-            launch_mv<9, MV_PLAIN>(s, g, A.as<double>(), act.as<int32_t>(), xu, xv, p.zu, p.zv,
-                                                            nullptr, nullptr, nullptr, nullptr, rc0);
+            launch_mv<9, MV_PLAIN>(s, g, matrix(), act.as<int32_t>(), xu, xv, p.zu, p.zv, nullptr, nullptr, nullptr,
+                                   nullptr, nullptr, rc0);
         k_resid_vec<<<nb, kBlock, 0, s>>>(g, act.as<int32_t>(), p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, rc1);
         CU(cudaGetLastError());
         CU(cudaMemcpyAsync(h_state, st, sizeof(SolveState), cudaMemcpyDeviceToHost, s));
@@ -995,7 +1008,7 @@ struct Solver {
         const size_t bs = (size_t)NC * nvec;
         double *A0 = A.as<double>();
         TRY(sym_check(L, A0, A0 + bs, A0 + 2 * bs, A0 + 3 * bs, maxdiff, nwarn));
-        if (is3d) mixed.stale = true;  // the FP32 copies follow the averaged matrix
+        if (is3d) matrix_changed();  // the copies follow the averaged matrix
         return CISMGPU_OK;
     }
 
@@ -1179,6 +1192,57 @@ struct Solver {
         return CISMGPU_OK;
     }
 
+    // A, or the array it lives in, has changed: the copies made from it are stale.
+    void matrix_changed() {
+        mixed.stale = true;
+        half_state = -1;
+    }
+
+    // No owned vertex lies on the edge of the array.
+    bool inner_geometry() const { return g.ilo >= 1 && g.ihi <= g.NX - 2 && g.jlo >= 1 && g.jhi <= g.NY - 2; }
+
+    // Test the 3D matrix for exact symmetry and build its half (k_half3d), once per matrix; a32
+    // receives the FP32 half as well.  Synchronizes the stream when it runs.
+    int half_setup(float4 *a32) {
+        half_state = 0;
+        const size_t bytes = (size_t)14 * nvec * 4 * sizeof(double);
+        CU(half.ensure(bytes + 256));
+        int *flag = reinterpret_cast<int *>(half.as<char>() + bytes);
+        CU(cudaMemsetAsync(flag, 0, sizeof(int), stream));
+        k_half3d<<<dim3(nblocks(g.NQ), (unsigned)g.nz, 14), kBlock, 0, stream>>>(
+            g, act.as<int32_t>(), A.as<double>(), half.as<double>(), a32, flag);
+        CU(cudaGetLastError());
+        int h = 1;
+        CU(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        CU(cudaStreamSynchronize(stream));
+        half_state = h == 0 ? 1 : 0;
+        return CISMGPU_OK;
+    }
+
+    // The matvecs of an FP64 solve read the symmetric half where that pays: a matrix that L2
+    // does not keep (kHalfMinBytes) and enough iterations for its test and copy.  A device without
+    // room for the copy reads the planes.
+    int matrix_setup(int maxiters) {
+        if (is3d) CU(terms.ensure((size_t)2 * nvec * sizeof(double)));
+        if (!is3d || half_state >= 0 || !inner_geometry() || maxiters < kHalfMinIters ||
+            (size_t)108 * nvec * sizeof(double) < kHalfMinBytes)
+            return CISMGPU_OK;
+        const int rc = half_setup(nullptr);
+        if (rc == CISMGPU_ENOMEM) {
+            (void)cudaGetLastError();
+            g_last_error.clear();
+            return CISMGPU_OK;
+        }
+        return rc;
+    }
+
+    // The matrix in the layout the matvecs read.
+    MvMatrix matrix() const {
+        MvMatrix M{A.as<double>(), half.as<double>(), MV_BOUNDS};
+        if (inner_geometry()) M.layout = (is3d && half_state == 1) ? MV_HALF : MV_INNER;
+        return M;
+    }
+
     // A pointwise statement group (Upd, and a pointwise preconditioner PRE) over every node.
     template <int UPD, int PRE = P_KEEP>
     void node(const double *dgu = nullptr, const double *dgv = nullptr) {
@@ -1356,18 +1420,20 @@ int Solver::run_standard(int precond, int ncheck, double tol, int maxiters) {
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const unsigned nb = nblocks(g.NQ);
     auto rc = [&](int epi, int iter) { return RedCtx{part, st, epi, iter}; };
     const Geom gg = g;
     prof_bytes = mv_bytes(0);
 
+    TRY(matrix_setup(maxiters));
+    const MvMatrix M = matrix();
+    double *T = terms.as<double>();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
     halo(p.xu, p.xv);
-    launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr,
-                                              nullptr, rc(EPI_NONE, 0));
+    launch_mv<NCC, MV_PLAIN>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr,
+                                              nullptr, T, rc(EPI_NONE, 0));
     node<U_STD_INIT>();
     k_dot_bb<<<nb, kBlock, 0, s>>>(gg, p.bu, p.bv, rc(EPI_L2RHS, 0));
     CU(cudaGetLastError());
@@ -1377,15 +1443,14 @@ int Solver::run_standard(int precond, int ncheck, double tol, int maxiters) {
         TRY((precond_step<NCC, true>(upd, precond, rc(EPI_STD_ETA1, iter))));
         node<U_DIR>();
         TRY(timed([&] {
-            launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr,
-                                                   nullptr, rc(EPI_STD_ETA2, iter));
+            launch_mv<NCC, MV_DQ>(s, gg, M, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr,
+                                                   nullptr, T, rc(EPI_STD_ETA2, iter));
         }));
         upd = U_XR;
         if (is_check(iter, ncheck)) {
             node<U_XR_X>();
             upd = U_NONE;
-            launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv,
-                                                      rc(EPI_CHECK, iter));
+            launch_mv<NCC, MV_RESID>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, T, rc(EPI_CHECK, iter));
             CU(cudaGetLastError());
             int f = poll.after_check();
             if (f < 0) return fail(CISMGPU_ECUDA, "polling the convergence flag failed");
@@ -1404,7 +1469,6 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const unsigned nb = nblocks(g.NQ);
     auto rc = [&](int epi, int iter) { return RedCtx{part, st, epi, iter}; };
@@ -1414,6 +1478,9 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     const bool tri = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
     if (tri && NCC == 9) maxiters = 100;
 
+    TRY(matrix_setup(maxiters));
+    const MvMatrix M = matrix();
+    double *T = terms.as<double>();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     // r = d = z = q = Az = 0 (:3048-3061)
@@ -1421,12 +1488,11 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     k_dot_bb<<<nb, kBlock, 0, s>>>(gg, p.bu, p.bv, rc(EPI_L2RHS, 0));
     // first pass (:3085-3290)
     halo(p.xu, p.xv);
-    launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr,
-                                              nullptr, rc(EPI_NONE, 1));
+    launch_mv<NCC, MV_PLAIN>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr,
+                                              nullptr, T, rc(EPI_NONE, 1));
     node<U_CG_INIT>();
     TRY((precond_step<NCC, true>(U_RHALO, precond, rc(EPI_CG_RHO0, 1), 1)));  // and the halo of r, d = z
-    launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr,
-                                           rc(EPI_CG_FIRST, 1));
+    launch_mv<NCC, MV_DQ>(s, gg, M, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, T, rc(EPI_CG_FIRST, 1));
     node<U_XR_Q>();  // the halo of q, x and r
     CU(cudaGetLastError());
     Poller poll(*this);
@@ -1435,14 +1501,13 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     for (int iter = 2; iter <= maxiters; ++iter) {
         TRY((precond_step<NCC, false>(upd, precond, rc(EPI_NONE, iter))));
         TRY(timed([&] {
-            launch_mv<NCC, MV_CG_AZ>(s, gg, Ad, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru,
-                                                      p.rv, rc(EPI_CG_ITER, iter));
+            launch_mv<NCC, MV_CG_AZ>(s, gg, M, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru,
+                                                      p.rv, T, rc(EPI_CG_ITER, iter));
         }));
         upd = U_CG;
         if (is_check(iter, ncheck)) {
             node<U_CG>();
-            launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv,
-                                                      rc(EPI_CHECK, iter));
+            launch_mv<NCC, MV_RESID>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, T, rc(EPI_CHECK, iter));
             upd = U_RHALO;  // with the next preconditioner
             CU(cudaGetLastError());
             int f = poll.after_check();
@@ -1467,16 +1532,18 @@ int Solver::run_standard_repro(int precond, int ncheck, double tol, int maxiters
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
     double S0 = 0.0;
 
+    TRY(matrix_setup(maxiters));
+    const MvMatrix M = matrix();
+    double *T = terms.as<double>();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
     halo(p.xu, p.xv);
-    launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
+    launch_mv<NCC, MV_PLAIN>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, T, none);
     node<U_STD_INIT>();
     CU(cudaGetLastError());
     TRY(repro_dot(p.bu, p.bu, p.bv, p.bv, &S0));
@@ -1486,7 +1553,7 @@ int Solver::run_standard_repro(int precond, int ncheck, double tol, int maxiters
         TRY(repro_dot(p.ru, p.zu, p.rv, p.zv, &S0));
         TRY(repro_epilogue(EPI_STD_ETA1, iter, S0, 0.0));
         node<U_DIR>();
-        launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
+        launch_mv<NCC, MV_DQ>(s, gg, M, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, T, none);
         CU(cudaGetLastError());
         TRY(repro_dot(p.du, p.qu, p.dv, p.qv, &S0));
         TRY(repro_epilogue(EPI_STD_ETA2, iter, S0, 0.0));
@@ -1495,7 +1562,7 @@ int Solver::run_standard_repro(int precond, int ncheck, double tol, int maxiters
             node<U_XR>();
         } else {
             node<U_XR_X>();
-            launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
+            launch_mv<NCC, MV_RESID>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, T, none);
             CU(cudaGetLastError());
             TRY(repro_dot(p.ru, p.ru, p.rv, p.rv, &S0));
             TRY(repro_epilogue(EPI_CHECK, iter, S0, 0.0));
@@ -1517,7 +1584,6 @@ int Solver::run_chrongear_repro(int precond, int ncheck, double tol, int maxiter
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
@@ -1525,6 +1591,9 @@ int Solver::run_chrongear_repro(int precond, int ncheck, double tol, int maxiter
     if (tri && NCC == 9) maxiters = 100;
     double S0 = 0.0, S1 = 0.0;
 
+    TRY(matrix_setup(maxiters));
+    const MvMatrix M = matrix();
+    double *T = terms.as<double>();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     CU(cudaMemsetAsync(p.ru, 0, (size_t)(VAZ_V - VR_U + 1) * nvec * sizeof(double), s));
@@ -1532,11 +1601,11 @@ int Solver::run_chrongear_repro(int precond, int ncheck, double tol, int maxiter
     TRY(repro_epilogue(EPI_L2RHS, 0, S0, 0.0));
     // first pass
     halo(p.xu, p.xv);
-    launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
+    launch_mv<NCC, MV_PLAIN>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, T, none);
     node<U_CG_INIT>();
     TRY((precond_step<NCC, false>(U_RHALO, precond, none)));
     CU(cudaMemcpyAsync(p.du, p.zu, (size_t)2 * nvec * sizeof(double), cudaMemcpyDeviceToDevice, s));  // d = z
-    launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
+    launch_mv<NCC, MV_DQ>(s, gg, M, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, T, none);
     CU(cudaGetLastError());
     TRY(repro_dot(p.ru, p.zu, p.rv, p.zv, &S0));
     TRY(repro_dot(p.du, p.qu, p.dv, p.qv, &S1));
@@ -1551,14 +1620,14 @@ int Solver::run_chrongear_repro(int precond, int ncheck, double tol, int maxiter
         if (done) break;
         TRY((precond_step<NCC, false>(upd, precond, none)));
         upd = U_NONE;
-        launch_mv<NCC, MV_CG_AZ>(s, gg, Ad, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru, p.rv, none);
+        launch_mv<NCC, MV_CG_AZ>(s, gg, M, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru, p.rv, T, none);
         CU(cudaGetLastError());
         TRY(repro_dot(p.ru, p.zu, p.rv, p.zv, &S0));
         TRY(repro_dot(p.Azu, p.zu, p.Azv, p.zv, &S1));
         TRY(repro_epilogue(EPI_CG_ITER, iter, S0, S1));
         node<U_CG>();
         if (is_check(iter, ncheck)) {
-            launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
+            launch_mv<NCC, MV_RESID>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, T, none);
             CU(cudaGetLastError());
             TRY(repro_dot(p.ru, p.ru, p.rv, p.rv, &S0));
             TRY(repro_epilogue(EPI_CHECK, iter, S0, 0.0));
@@ -1580,16 +1649,18 @@ int Solver::run_standard_seq(int precond, int ncheck, double tol, int maxiters) 
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
     prof_bytes = mv_bytes(0);
 
+    TRY(matrix_setup(maxiters));
+    const MvMatrix M = matrix();
+    double *T = terms.as<double>();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
     halo(p.xu, p.xv);
-    launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
+    launch_mv<NCC, MV_PLAIN>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, T, none);
     node<U_STD_INIT>();
     CU(cudaGetLastError());
     TRY(seq_dot(p.bu, p.bu, p.bv, p.bv, EPI_L2RHS, 0));
@@ -1599,14 +1670,14 @@ int Solver::run_standard_seq(int precond, int ncheck, double tol, int maxiters) 
         TRY(seq_dot(p.ru, p.zu, p.rv, p.zv, EPI_STD_ETA1, iter));
         node<U_DIR>();
         TRY(timed([&] {
-            launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
+            launch_mv<NCC, MV_DQ>(s, gg, M, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, T, none);
         }));
         TRY(seq_dot(p.du, p.qu, p.dv, p.qv, EPI_STD_ETA2, iter));
         if (!is_check(iter, ncheck)) {
             node<U_XR>();
         } else {
             node<U_XR_X>();
-            launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
+            launch_mv<NCC, MV_RESID>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, T, none);
             TRY(seq_dot(p.ru, p.ru, p.rv, p.rv, EPI_CHECK, iter));
             int f = poll.after_check();
             if (f < 0) return fail(CISMGPU_ECUDA, "polling the convergence flag failed");
@@ -1626,7 +1697,6 @@ int Solver::run_chrongear_seq(int precond, int ncheck, double tol, int maxiters)
     SolveState *st = state.as<SolveState>();
     DD *part = partials.as<DD>();
     const Ptrs p = ptrs();
-    const double *Ad = A.as<double>();
     const int32_t *ac = act.as<int32_t>();
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
@@ -1634,17 +1704,20 @@ int Solver::run_chrongear_seq(int precond, int ncheck, double tol, int maxiters)
     const bool tri = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
     if (tri && NCC == 9) maxiters = 100;
 
+    TRY(matrix_setup(maxiters));
+    const MvMatrix M = matrix();
+    double *T = terms.as<double>();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     CU(cudaMemsetAsync(p.ru, 0, (size_t)(VAZ_V - VR_U + 1) * nvec * sizeof(double), s));
     TRY(seq_dot(p.bu, p.bu, p.bv, p.bv, EPI_L2RHS, 0));
     // first pass
     halo(p.xu, p.xv);
-    launch_mv<NCC, MV_PLAIN>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, none);
+    launch_mv<NCC, MV_PLAIN>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, nullptr, nullptr, nullptr, nullptr, T, none);
     node<U_CG_INIT>();
     TRY((precond_step<NCC, false>(U_RHALO, precond, none)));
     CU(cudaMemcpyAsync(p.du, p.zu, (size_t)2 * nvec * sizeof(double), cudaMemcpyDeviceToDevice, s));  // d = z
-    launch_mv<NCC, MV_DQ>(s, gg, Ad, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, none);
+    launch_mv<NCC, MV_DQ>(s, gg, M, ac, p.du, p.dv, p.qu, p.qv, nullptr, nullptr, nullptr, nullptr, T, none);
     TRY(seq_dot2(p.ru, p.zu, p.rv, p.zv, p.du, p.qu, p.dv, p.qv, EPI_CG_RHO0, EPI_CG_FIRST, 1));
     node<U_XR_Q>();  // the halo of q, x and r
     CU(cudaGetLastError());
@@ -1654,12 +1727,12 @@ int Solver::run_chrongear_seq(int precond, int ncheck, double tol, int maxiters)
         TRY((precond_step<NCC, false>(upd, precond, none)));
         upd = U_NONE;
         TRY(timed([&] {
-            launch_mv<NCC, MV_CG_AZ>(s, gg, Ad, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru, p.rv, none);
+            launch_mv<NCC, MV_CG_AZ>(s, gg, M, ac, p.zu, p.zv, p.Azu, p.Azv, nullptr, nullptr, p.ru, p.rv, T, none);
         }));
         TRY(seq_dot2(p.ru, p.zu, p.rv, p.zv, p.Azu, p.zu, p.Azv, p.zv, EPI_CG_ITER, EPI_NONE, iter));
         node<U_CG>();
         if (is_check(iter, ncheck)) {
-            launch_mv<NCC, MV_RESID>(s, gg, Ad, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, none);
+            launch_mv<NCC, MV_RESID>(s, gg, M, ac, p.xu, p.xv, p.zu, p.zv, p.bu, p.bv, p.ru, p.rv, T, none);
             TRY(seq_dot(p.ru, p.ru, p.rv, p.rv, EPI_CHECK, iter));
             upd = U_RHALO;  // with the next preconditioner
             CU(cudaGetLastError());
@@ -1716,7 +1789,7 @@ static MDesc mixed_desc(const Solver &sv, int precond, int TY) {  // TY: the sol
     D.ntiles = D.tiles_x * D.tiles_y;
     D.A32 = m.A32;
     D.A64 = sv.A.as<double>();
-    D.A64i = (m.sym || m.il) ? m.A64i : nullptr;
+    D.A64i = m.sym ? sv.half.as<double2>() : (m.il ? m.A64i : nullptr);
     D.sym = m.sym ? 1 : 0;
     D.pre = m.pre;
     D.act = sv.act.as<int32_t>();
@@ -1853,10 +1926,9 @@ static int mixed_prepare(Solver &sv, int precond, int TY) {
             return dev_alloc(p, n);
         };
         CU(alloc((void **)&m.A32, (size_t)NC * nvec * sizeof(float4)));
-        // the interleaved FP64 copy: for a streamed matrix, and in 3D for the symmetric half
-        if (NC == 27 || (size_t)NC * (size_t)nvec * sizeof(float4) > kStreamBytes)
+        // 2D: the interleaved FP64 copy of a streamed matrix (3D: below)
+        if (NC == 9 && (size_t)NC * (size_t)nvec * sizeof(float4) > kStreamBytes)
             CU(alloc((void **)&m.A64i, (size_t)NC * nvec * 2 * sizeof(double2)));
-        CU(alloc((void **)&m.flag, 256));
         CU(alloc((void **)&m.pre, (size_t)6 * nvec * sizeof(float)));
         CU(alloc((void **)&m.vec, (size_t)16 * nvec * sizeof(float)));
         CU(alloc((void **)&m.state, sizeof(MState)));
@@ -1872,23 +1944,27 @@ static int mixed_prepare(Solver &sv, int precond, int TY) {
         m.ntiles = 0;
     }
     if (m.stale) {  // new matrix: FP32 copy (couplings leaving the grid set to zero)
-        // 3D: an exactly symmetric matrix is stored as its symmetric half (14 of 27 couplings)
+        // 3D: an exactly symmetric matrix is stored as its symmetric half (14 of 27 couplings), the
+        // FP64 half shared with the FP64 solvers; any other as the full interleaved copy (the check
+        // steps read it with the x tile in shared memory)
         m.sym = false;
-        if (NC == 27) {
-            CU(cudaMemsetAsync(m.flag, 0, sizeof(int), sv.stream));
-            k_sym_exact3d<<<nblocks(g.NQ), kBlock, 0, sv.stream>>>(g, sv.act.as<int32_t>(), sv.A.as<double>(), m.flag);
-            CU(cudaGetLastError());
-            int hflag = 1;
-            CU(cudaMemcpyAsync(&hflag, m.flag, sizeof(int), cudaMemcpyDeviceToHost, sv.stream));
-            CU(cudaStreamSynchronize(sv.stream));
-            m.sym = hflag == 0 && !g_mixed_full_storage.load();
+        if (NC == 27 && sv.inner_geometry() && !g_mixed_full_storage.load()) {
+            const int rc = sv.half_setup(m.A32);
+            if (rc && rc != CISMGPU_ENOMEM) return rc;
+            (void)cudaGetLastError();
+            m.sym = rc == CISMGPU_OK && sv.half_state == 1;
         }
-        // the interleaved FP64 copy: always in 3D (the check steps read it with the x tile in
-        // shared memory), in 2D for a streamed matrix
-        m.il = !m.sym && m.A64i != nullptr && (NC == 27 || (size_t)NC * (size_t)nvec * sizeof(float4) > kStreamBytes);
-        if (m.sym) k_to_half<<<1184, kBlock, 0, sv.stream>>>(g, sv.A.as<double>(), m.A32, m.A64i);
-        else if (NC == 27) k_to_f32<27><<<1184, kBlock, 0, sv.stream>>>(g, sv.A.as<double>(), m.A32, m.il ? m.A64i : nullptr);
-        else k_to_f32<9><<<1184, kBlock, 0, sv.stream>>>(g, sv.A.as<double>(), m.A32, m.A64i);
+        if (NC == 27 && !m.sym) {
+            sv.half.release();
+            sv.half_state = 0;
+            if (!m.A64i) {
+                CU(dev_alloc((void **)&m.A64i, (size_t)NC * nvec * 2 * sizeof(double2)));
+                m.nbytes += (size_t)NC * nvec * 2 * sizeof(double2);
+            }
+        }
+        m.il = !m.sym && m.A64i != nullptr;
+        if (NC == 27 && !m.sym) k_to_f32<27><<<1184, kBlock, 0, sv.stream>>>(g, sv.A.as<double>(), m.A32, m.A64i);
+        else if (NC == 9) k_to_f32<9><<<1184, kBlock, 0, sv.stream>>>(g, sv.A.as<double>(), m.A32, m.A64i);
         CU(cudaGetLastError());
         m.stale = false;
         m.precond = -1;
@@ -2404,13 +2480,11 @@ static int oneshot_matvec(bool is3d, int nx, int ny, int nz, const cismgpu_par_t
     k_init_state<<<1, 1, 0, sv.stream>>>(st, 0.0, 0);
     RedCtx rc0{sv.partials.as<DD>(), st, EPI_NONE, 0};
     if (is3d)
-        launch_mv<27, MV_PLAIN>(sv.stream, sv.g, sv.A.as<double>(), sv.act.as<int32_t>(),
-                                                                      p.bu, p.bv, p.xu, p.xv, nullptr, nullptr,
-                                                                      nullptr, nullptr, rc0);
+        launch_mv<27, MV_PLAIN>(sv.stream, sv.g, sv.matrix(), sv.act.as<int32_t>(), p.bu, p.bv, p.xu, p.xv, nullptr,
+                                nullptr, nullptr, nullptr, nullptr, rc0);
     else
-        launch_mv<9, MV_PLAIN>(sv.stream, sv.g, sv.A.as<double>(), sv.act.as<int32_t>(),
-                                                                     p.bu, p.bv, p.xu, p.xv, nullptr, nullptr,
-                                                                     nullptr, nullptr, rc0);
+        launch_mv<9, MV_PLAIN>(sv.stream, sv.g, sv.matrix(), sv.act.as<int32_t>(), p.bu, p.bv, p.xu, p.xv, nullptr,
+                                nullptr, nullptr, nullptr, nullptr, rc0);
     CU(cudaGetLastError());
     return sv.download(VX_U, VX_V, yu, yv);
 }
@@ -2458,7 +2532,7 @@ static int oneshot_symmetry(bool is3d, int nx, int ny, int nz, const cismgpu_par
     CU(cudaMemcpyAsync(sv.act.p, act, (size_t)g.NQ * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     const size_t bs = (size_t)sv.NC * sv.nvec;
     CU(sv.A.ensure(4 * bs * sizeof(double)));
-    sv.mixed.stale = true;  // the matrix buffer holds the caller's layout until the next upload
+    sv.matrix_changed();  // the matrix buffer holds the caller's layout until the next upload
     double *A0 = sv.A.as<double>();
     for (int b = 0; b < 4; ++b)
         CU(cudaMemcpyAsync(A0 + b * bs, blocks[b], bs * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -2518,7 +2592,7 @@ static int oneshot_assemble(bool three_d, int nx, int ny, int nz, int nhalo, con
     TRY(sv.set_geom(make_geom(nx, ny, three_d ? nz : 1, &par), three_d));
     const size_t bs = (size_t)NC * sv.nvec;
     CU(sv.A.ensure(4 * bs * sizeof(double)));
-    sv.mixed.stale = true;  // the matrix buffer holds the caller's layout until the next upload
+    sv.matrix_changed();  // the matrix buffer holds the caller's layout until the next upload
     double *A0 = sv.A.as<double>();
     SymIdx L{};
     for (int c = 0; c < 27; ++c) L.map[c] = c < NC ? indx[c] : 1;
@@ -3187,7 +3261,7 @@ static int oneshot_boundary3d(int which, int nx, int ny, int nz, int nhalo, doub
     TRY(sv.set_geom(make_geom(nx, ny, nz, &par), true));
     const size_t bs = (size_t)27 * sv.nvec;
     CU(sv.A.ensure(4 * bs * sizeof(double)));
-    sv.mixed.stale = true;  // the matrix buffer holds the caller's layout until the next upload
+    sv.matrix_changed();  // the matrix buffer holds the caller's layout until the next upload
     double *A0 = sv.A.as<double>();
     double *blk[4] = {A0, A0 + bs, A0 + 2 * bs, A0 + 3 * bs};
     double *host[4] = {Auu, Auv, Avu, Avv};
@@ -3254,7 +3328,7 @@ static int oneshot_boundary2d(int which, int nx, int ny, int nhalo, double dx, d
     TRY(sv.set_geom(make_geom(nx, ny, 1, &par), false));
     const size_t bs = (size_t)9 * sv.nvec;
     CU(sv.A.ensure(4 * bs * sizeof(double)));
-    sv.mixed.stale = true;
+    sv.matrix_changed();
     double *A0 = sv.A.as<double>();
     double *blk[4] = {A0, A0 + bs, A0 + 2 * bs, A0 + 3 * bs};
     double *host[4] = {Auu, Auv, Avu, Avv};
@@ -3313,7 +3387,7 @@ static int oneshot_assemble_diva(int nx, int ny, int nz, int nhalo, const double
     TRY(sv.set_geom(make_geom(nx, ny, 1, &par), false));
     const size_t bs = (size_t)9 * sv.nvec, neq = (size_t)(nz - 1) * 4 * nx * ny;
     CU(sv.A.ensure(4 * bs * sizeof(double)));
-    sv.mixed.stale = true;
+    sv.matrix_changed();
     CU(sv.diva_eq[0].ensure(neq * sizeof(double)));
     CU(sv.diva_eq[1].ensure(neq * sizeof(double)));
     sv.diva_valid = false;  // the one-shot solver's state buffers hold the caller's state only
@@ -3415,7 +3489,7 @@ static int solver_assemble(cismgpu_solver_t *h, bool three_d, int nzl, int nhalo
     L.raw3 = 0;
     const size_t bs = (size_t)sv.NC * sv.nvec;
     double *A0 = sv.A.as<double>();
-    sv.mixed.stale = true;  // the FP32 copies follow the new matrix
+    sv.matrix_changed();  // the FP32 copies follow the new matrix
     return sv.assemble(three_d, nzl, L, A0, A0 + bs, A0 + 2 * bs, A0 + 3 * bs, nhalo, sigma, active_cell, xVertex,
                        yVertex, uvel, vvel, sv.x_current ? VX_U : VX0_U, stagusrf, stagthck, flwafact, whichapprox,
                        whichefvs, efvs_constant, effstrain_min, n_glen, efvs);
@@ -3506,7 +3580,7 @@ int cismgpu_solver_assemble_system_3d(cismgpu_solver_t *h, int nhalo, double dx,
     k_halo<<<hb, kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));
-    sv.mixed.stale = true;
+    sv.matrix_changed();
     return CISMGPU_OK;
 }
 
@@ -3586,7 +3660,7 @@ int cismgpu_solver_assemble_system_2d(cismgpu_solver_t *h, int nz, int nhalo, do
     k_halo<<<hb, kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));
-    sv.mixed.stale = true;
+    sv.matrix_changed();
     return CISMGPU_OK;
 }
 
@@ -3644,7 +3718,7 @@ int cismgpu_solver_assemble_stiffness_2d_diva(cismgpu_solver_t *h, int nz, int n
     L.raw3 = 0;
     const size_t bs = (size_t)9 * sv.nvec;
     double *A0 = sv.A.as<double>();
-    sv.mixed.stale = true;
+    sv.matrix_changed();
     TRY(sv.assemble_diva(nz, L, A0, A0 + bs, A0 + 2 * bs, A0 + 3 * bs, nhalo, sigma, stagsigma, active_cell, xVertex,
                          yVertex, uvel_2d, vvel_2d, sv.x_current ? VX_U : VX0_U, stagthck, thck, btractx, btracty,
                          diva_slope_factor_x, diva_slope_factor_y, flwafact, whichefvs, efvs_constant, effstrain_min,
@@ -3700,7 +3774,7 @@ int cismgpu_solver_assemble_system_2d_diva(
     k_halo<<<hb, kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));
-    sv.mixed.stale = true;
+    sv.matrix_changed();
     return CISMGPU_OK;
 }
 
@@ -3741,7 +3815,7 @@ int cismgpu_solver_restore(cismgpu_solver_t *h) {
     CU(cudaMemcpyAsync(sv.A.p, sv.A_sav.p, abytes, cudaMemcpyDeviceToDevice, sv.stream));
     CU(cudaMemcpyAsync(p.x0u, sv.x_sav.p, xbytes, cudaMemcpyDeviceToDevice, sv.stream));
     CU(cudaStreamSynchronize(sv.stream));
-    sv.mixed.stale = true;  // the FP32 copies follow the restored matrix
+    sv.matrix_changed();  // the FP32 copies follow the restored matrix
     sv.x_current = false;   // the current velocity is the saved one, and the next solve starts from it
     return CISMGPU_OK;
 }
@@ -3778,7 +3852,8 @@ int cismgpu_solver_profile_read(cismgpu_solver_t *h, double *total_ms, int *laun
 size_t cismgpu_solver_device_bytes(const cismgpu_solver_t *h) {
     if (!h) return 0;
     const Solver &s = h->sv;
-    return s.A.n + s.raw.n + s.vec.n + s.act.n + s.partials.n + s.state.n + s.map.n + s.mixed.bytes();
+    return s.A.n + s.raw.n + s.vec.n + s.act.n + s.partials.n + s.state.n + s.map.n + s.half.n + s.terms.n +
+           s.sia.n + s.mixed.bytes();
 }
 
 int cismgpu_solver_destroy(cismgpu_solver_t *h) {

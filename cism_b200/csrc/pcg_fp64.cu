@@ -158,135 +158,172 @@ __device__ __forceinline__ void col_of(const Geom &g, long long q, int &i, int &
 // ---------------------------------------------------------------------------
 // structured matvec row (matvec_multiply_structured_3d :5612-5650, _2d :5739-5771)
 // ---------------------------------------------------------------------------
-template <int NC>
-__device__ __forceinline__ void mv_row(const Geom &g, const double *__restrict__ A, const double *__restrict__ xu,
+// The matrix as a matvec reads it.
+//   MV_BOUNDS: the coefficient planes, every coupling tested against the array (any geometry);
+//   MV_INNER: the same planes, no owned vertex on the edge of the array, so that only the levels
+//     are tested, which is uniform over a block: all loads of a row are issued without branches;
+//   MV_HALF: MV_INNER of an exactly symmetric 3D matrix (as the reference's check leaves it): its
+//     symmetric half of k_half3d, one 32-byte load per coupling and node.  A lower coupling c is
+//     its partner's coupling 26 - c with uv and vu swapped, the same number, so the sums are too.
+// 3D product on 201x201x11: 72.7 us with tests, 59.7 without, 37.0 from the half (5.6 TB/s; it
+// streams 448 bytes a node instead of 864, and the partners' couplings come from L2).
+enum MvLayout { MV_BOUNDS = 0, MV_INNER, MV_HALF };
+
+struct MvMatrix {
+    const double *A;   // [4][NC][nz][NQ]
+    const double *H;   // MV_HALF: [14][nz][NQ][4], couplings 13..26 as (uu, uv, vu, vv)
+    int layout;
+};
+
+struct __align__(32) Dbl4 { double x, y, z, w; };
+__device__ __forceinline__ Dbl4 ldg256(const double *p) {  // 32-byte aligned, read-only in the launch
+    Dbl4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
+template <int NC, int LAY>
+__device__ __forceinline__ void mv_row(const Geom &g, const MvMatrix &M, const double *__restrict__ xu,
                                        const double *__restrict__ xv, int i, int j, long long q, int k,
                                        double &yu, double &yv) {
-    const long long plane = (long long)g.nz * g.NQ;
-    const double *Auu = A, *Auv = A + NC * plane, *Avu = A + 2 * NC * plane, *Avv = A + 3 * NC * plane;
+    const long long plane = (long long)g.nz * g.NQ, e = (long long)k * g.NQ + q;
+    const double *__restrict__ Auu = M.A, *__restrict__ Auv = M.A + NC * plane, *__restrict__ Avu = M.A + 2 * NC * plane,
+                              *__restrict__ Avv = M.A + 3 * NC * plane;
+    constexpr int K0 = (NC == 27) ? -1 : 0, K1 = (NC == 27) ? 1 : 0;
     double su = 0.0, sv = 0.0;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const int iA = c % 3 - 1, jA = (c / 3) % 3 - 1, kA = (NC == 27) ? c / 9 - 1 : 0;
-        if (k + kA >= 0 && k + kA < g.nz && i + iA >= 0 && i + iA < g.NX && j + jA >= 0 && j + jA < g.NY) {
-            const long long a = (long long)c * plane + (long long)k * g.NQ + q;
-            const long long n = (long long)(k + kA) * g.NQ + q + iA + (long long)jA * g.NX;
+    for (int kA = K0; kA <= K1; ++kA) {
+        if (k + kA < 0 || k + kA >= g.nz) continue;
+#pragma unroll
+        for (int c9 = 0; c9 < 9; ++c9) {
+            const int iA = c9 % 3 - 1, jA = c9 / 3 - 1, c = (kA - K0) * 9 + c9;
+            if (LAY == MV_BOUNDS && (i + iA < 0 || i + iA >= g.NX || j + jA < 0 || j + jA >= g.NY)) continue;
+            const long long n = e + (long long)kA * g.NQ + (long long)jA * g.NX + iA;
             const double x1 = xu[n], x2 = xv[n];
-            su = __dadd_rn(__dadd_rn(su, __dmul_rn(Auu[a], x1)), __dmul_rn(Auv[a], x2));
-            sv = __dadd_rn(__dadd_rn(sv, __dmul_rn(Avu[a], x1)), __dmul_rn(Avv[a], x2));
+            Dbl4 a;
+            if (LAY == MV_HALF) {
+                if (c >= 13) {
+                    a = ldg256(M.H + 4 * ((c - 13) * plane + e));
+                } else {
+                    const Dbl4 p = ldg256(M.H + 4 * ((13 - c) * plane + n));
+                    a = Dbl4{p.x, p.z, p.y, p.w};
+                }
+            } else {
+                const long long f = c * plane + e;
+                a = Dbl4{__ldg(Auu + f), __ldg(Auv + f), __ldg(Avu + f), __ldg(Avv + f)};
+            }
+            su = __dadd_rn(__dadd_rn(su, __dmul_rn(a.x, x1)), __dmul_rn(a.y, x2));
+            sv = __dadd_rn(__dadd_rn(sv, __dmul_rn(a.z, x1)), __dmul_rn(a.w, x2));
         }
     }
     yu = su;
     yv = sv;
 }
 
+// The symmetric half of a 3D matrix, [14][nz][NQ][4]: couplings c = 13..26 (the diagonal and the
+// upper offsets) of every node as (uu, uv, vu, vv), couplings leaving the array as zero.  *flag is
+// set if a lower coupling of an owned active row differs from its transpose partner (Auu with
+// Auu, Auv with Avu, Avv with Avv, bit for bit), which check_symmetry_assembled_matrix_3d averages
+// to equality before every 3D solve (glissade_velo_higher.F90:2923-2931).  No owned vertex may lie
+// on the edge of the array (a partner is then always inside).  a32 (may be null): the same half
+// as FP32.  One thread per node and stored coupling; every plane is read once, coalesced: 201x201x11
+// 98 us for the test and the FP64 half, where the mixed solver's test with one thread per column and its
+// copy took 299 + 93 us.
+__global__ void __launch_bounds__(kBlock) k_half3d(Geom g, const int32_t *__restrict__ act, const double *__restrict__ A,
+                                                   double *__restrict__ H, float4 *__restrict__ a32, int *flag) {
+    const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
+    const int k = blockIdx.y, h = blockIdx.z, c = 13 + h;
+    bool bad = false;
+    if (q < g.NQ) {
+        const int i = (int)(q % g.NX), j = (int)(q / g.NX);
+        const int iA = c % 3 - 1, jA = (c / 3) % 3 - 1, kA = c / 9 - 1;
+        const int in = i + iA, jn = j + jA;
+        const bool inside = in >= 0 && in < g.NX && jn >= 0 && jn < g.NY && k + kA < g.nz;
+        const long long plane = (long long)g.nz * g.NQ, bs = 27 * plane, e = (long long)k * g.NQ + q, f = c * plane + e;
+        Dbl4 a{0.0, 0.0, 0.0, 0.0};
+        if (inside) {
+            a = Dbl4{A[f], A[bs + f], A[2 * bs + f], A[3 * bs + f]};
+            const long long qn = (long long)jn * g.NX + in;
+            if (h > 0 && owned(g, in, jn) && act[qn] != 0) {
+                const long long l = (26 - c) * plane + (long long)(k + kA) * g.NQ + qn;
+                bad = A[l] != a.x || A[bs + l] != a.z || A[2 * bs + l] != a.y || A[3 * bs + l] != a.w;
+            }
+        }
+        reinterpret_cast<Dbl4 *>(H)[h * plane + e] = a;
+        if (a32) a32[h * plane + e] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
+    }
+    if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
+}
+
 enum MvMode { MV_PLAIN = 0, MV_RESID, MV_DQ, MV_CG_AZ };
 
 constexpr int kDotChunk = 8;  // levels whose loads a column's dot terms issue together
-
-// The dot terms of column q (modes with dot products), added over k in level order: a chunk's
-// loads together, then its terms in order.  Loads through L2 (__ldcg): the other levels' y and
-// r were written by other CTAs of the same launch.
-template <int MODE>
-__device__ __forceinline__ void col_dots(const Geom &g, long long q, const double *__restrict__ xu,
-                                         const double *__restrict__ xv, const double *__restrict__ yu,
-                                         const double *__restrict__ yv, const double *__restrict__ ru,
-                                         const double *__restrict__ rv, DD &s0, DD &s1) {
-    for (int k0 = 0; k0 < g.nz; k0 += kDotChunk) {
-        double t0[kDotChunk], t1[kDotChunk];
-#pragma unroll
-        for (int u = 0; u < kDotChunk; ++u) {
-            t0[u] = t1[u] = 0.0;
-            if (k0 + u >= g.nz) continue;
-            const long long e = (long long)(k0 + u) * g.NQ + q;
-            if (MODE == MV_RESID) {
-                const double r1 = __ldcg(ru + e), r2 = __ldcg(rv + e);
-                t0[u] = __dadd_rn(__dmul_rn(r1, r1), __dmul_rn(r2, r2));
-            } else if (MODE == MV_DQ) {
-                t0[u] = __dadd_rn(__dmul_rn(__ldcg(xu + e), __ldcg(yu + e)), __dmul_rn(__ldcg(xv + e), __ldcg(yv + e)));
-            } else if (MODE == MV_CG_AZ) {
-                const double z1 = __ldcg(xu + e), z2 = __ldcg(xv + e);
-                t0[u] = __dadd_rn(__dmul_rn(__ldcg(ru + e), z1), __dmul_rn(__ldcg(rv + e), z2));
-                t1[u] = __dadd_rn(__dmul_rn(__ldcg(yu + e), z1), __dmul_rn(__ldcg(yv + e), z2));
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kDotChunk; ++u)
-            if (k0 + u < g.nz) {
-                s0 = dd_add_d(s0, t0[u]);
-                if (MODE == MV_CG_AZ) s1 = dd_add_d(s1, t1[u]);
-            }
-    }
-}
 
 // y = A x over owned active columns, 0 elsewhere; optional fused statements:
 //   MV_RESID : r = b - y (whole array); S0 = (r,r)             [:1454-1466, :3504-3516]
 //   MV_DQ    : S0 = (x,y) with x = d, y = q                    [:1376-1381, :3241-3248]
 //   MV_CG_AZ : S0 = (r,z), S1 = (y,z) with x = z, y = Az       [:3401-3413]
-// k_mv_nodes: one thread per node (column q, level k = blockIdx.y), y = A x with the
-// reference's statements (mv_row), and for MV_RESID also r = b - y: every (column, level) is
-// independent, so a launch has nz * NQ/256 CTAs and enough loads in flight to stream the 108
-// coefficient planes.  Dot products in 3D: the last level block of each column block to
-// finish has one thread per column add its terms over k in level order (col_dots), then the
-// block tree of the 256 columns and the last-CTA tree: the order the reduction has always
-// had.  In 2D a column has one level, so every block adds its terms and reduces.
-template <int NC, int MODE>
-__global__ void __launch_bounds__(kBlock, 4) k_mv_nodes(Geom g, const double *__restrict__ A,
-                                                     const int32_t *__restrict__ act,
-                                                     const double *__restrict__ xu, const double *__restrict__ xv,
-                                                     double *__restrict__ yu, double *__restrict__ yv,
-                                                     const double *__restrict__ bu, const double *__restrict__ bv,
-                                                     double *__restrict__ ru, double *__restrict__ rv, RedCtx rc) {
-    // 2D (one level per column): the column's dot terms and the reduction in this kernel
-    constexpr bool FUSED = (NC == 9) && (MODE == MV_RESID || MODE == MV_DQ || MODE == MV_CG_AZ);
+// One thread per node (column q, level k = blockIdx.y): a launch has nz * NQ/256 CTAs and enough
+// loads in flight to stream the coefficients.  Dot products in 3D: every node writes its
+// term(s) to T ([2][nz][NQ]); the last level block of each column block to finish has one thread
+// per column add them over k in level order, then the block tree of the 256 columns and the
+// last-CTA tree: the order the reduction has always had, without a launch of its own, and with the
+// sums of the early column blocks overlapping the rest of the matvec.  The per-column-block
+// counters sit after the partials and return to zero here.  In 2D a column has one level, so
+// every block reduces its own terms.
+template <int NC, int MODE, int LAY>
+__global__ void __launch_bounds__(kBlock, 3) k_mv_nodes(Geom g, MvMatrix M, const int32_t *__restrict__ act,
+                                                        const double *__restrict__ xu, const double *__restrict__ xv,
+                                                        double *__restrict__ yu, double *__restrict__ yv,
+                                                        const double *__restrict__ bu, const double *__restrict__ bv,
+                                                        double *__restrict__ ru, double *__restrict__ rv,
+                                                        double *__restrict__ T, RedCtx rc) {
+    constexpr int NF = (MODE == MV_CG_AZ) ? 2 : 1;
     if (rc.st && rc.st->done) return;
     const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
     const int k = blockIdx.y;
-    DD s0{0.0, 0.0}, s1{0.0, 0.0};
+    const long long plane = (long long)g.nz * g.NQ;
+    bool own = false;
+    double t0 = 0.0, t1 = 0.0;
     if (q < g.NQ) {
         int i, j;
         col_of(g, q, i, j);
-        const bool own = owned(g, i, j);
-        const bool on = own && act[q] != 0;
+        own = owned(g, i, j);
         const long long e = (long long)k * g.NQ + q;
         double a = 0.0, b = 0.0;
-        if (on) mv_row<NC>(g, A, xu, xv, i, j, q, k, a, b);
+        if (own && act[q] != 0) mv_row<NC, LAY>(g, M, xu, xv, i, j, q, k, a, b);
         yu[e] = a;
         yv[e] = b;
-        double r1 = 0.0, r2 = 0.0;
         if (MODE == MV_RESID) {
-            r1 = __dsub_rn(bu[e], a);
-            r2 = __dsub_rn(bv[e], b);
+            const double r1 = __dsub_rn(bu[e], a), r2 = __dsub_rn(bv[e], b);
             ru[e] = r1;
             rv[e] = r2;
+            t0 = __dadd_rn(__dmul_rn(r1, r1), __dmul_rn(r2, r2));
+        } else if (MODE == MV_DQ && own) {
+            t0 = __dadd_rn(__dmul_rn(xu[e], a), __dmul_rn(xv[e], b));
+        } else if (MODE == MV_CG_AZ && own) {
+            const double z1 = xu[e], z2 = xv[e];
+            t0 = __dadd_rn(__dmul_rn(ru[e], z1), __dmul_rn(rv[e], z2));
+            t1 = __dadd_rn(__dmul_rn(a, z1), __dmul_rn(b, z2));
         }
-        if (FUSED && own) {
-            if (MODE == MV_RESID) {
-                s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(r1, r1), __dmul_rn(r2, r2)));
-            } else if (MODE == MV_DQ) {
-                s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(xu[e], a), __dmul_rn(xv[e], b)));
-            } else if (MODE == MV_CG_AZ) {
-                const double z1 = xu[e], z2 = xv[e];
-                s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(ru[e], z1), __dmul_rn(rv[e], z2)));
-                s1 = dd_add_d(s1, __dadd_rn(__dmul_rn(a, z1), __dmul_rn(b, z2)));
-            }
+        if (NC == 27 && MODE != MV_PLAIN && own) {
+            T[e] = t0;
+            if (NF > 1) T[plane + e] = t1;
         }
     }
-    if (FUSED) {
-        if (MODE == MV_CG_AZ) reduce_and_finish<2>(rc, s0, s1);
-        else reduce_and_finish<1>(rc, s0, s1);
-    }
-    if (NC == 27 && MODE != MV_PLAIN) {
-        // the last of the gridDim.y level blocks of column block blockIdx.x to finish adds the
-        // dot terms of its 256 columns over all levels, then the block tree and the last-CTA
-        // tree: the same order as a separate dot pass, without its launch and with the sums of
-        // the early column blocks overlapping the rest of the matvec.  The per-column-block
-        // counters sit after the partials and return to zero here.
+    if (MODE == MV_PLAIN) return;
+    DD s0{0.0, 0.0}, s1{0.0, 0.0};
+    if (NC == 9) {
+        if (own) {
+            s0 = dd_add_d(s0, t0);
+            if (NF > 1) s1 = dd_add_d(s1, t1);
+        }
+    } else {
         __shared__ bool lastk;
         __syncthreads();
         if (threadIdx.x == 0) {
             unsigned *cnt = reinterpret_cast<unsigned *>(rc.partials + 2 * gridDim.x) + blockIdx.x;
-            __threadfence();  // this block's y and r before its count
+            __threadfence();  // this block's terms before its count
             const unsigned t = atomicAdd(cnt, 1u);
             lastk = t == gridDim.y - 1;
             if (lastk) *cnt = 0u;
@@ -294,24 +331,38 @@ __global__ void __launch_bounds__(kBlock, 4) k_mv_nodes(Geom g, const double *__
         __syncthreads();
         if (!lastk) return;
         __threadfence();
-        DD d0{0.0, 0.0}, d1{0.0, 0.0};
-        if (q < g.NQ) {
-            int i, j;
-            col_of(g, q, i, j);
-            if (owned(g, i, j)) col_dots<MODE>(g, q, xu, xv, yu, yv, ru, rv, d0, d1);
-        }
-        if (MODE == MV_CG_AZ) reduce_and_finish<2>(rc, d0, d1);
-        else reduce_and_finish<1>(rc, d0, d1);
+        if (own)
+            for (int k0 = 0; k0 < g.nz; k0 += kDotChunk) {  // through L2: other CTAs of the launch wrote them
+                double v0[kDotChunk], v1[kDotChunk];
+#pragma unroll
+                for (int u = 0; u < kDotChunk; ++u) {
+                    const long long e = (long long)(k0 + u) * g.NQ + q;
+                    v0[u] = (k0 + u < g.nz) ? __ldcg(T + e) : 0.0;
+                    v1[u] = (NF > 1 && k0 + u < g.nz) ? __ldcg(T + plane + e) : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < kDotChunk; ++u)
+                    if (k0 + u < g.nz) {
+                        s0 = dd_add_d(s0, v0[u]);
+                        if (NF > 1) s1 = dd_add_d(s1, v1[u]);
+                    }
+            }
     }
+    reduce_and_finish<NF>(rc, s0, s1);
 }
 
-// y = A x (+ the statement MODE fuses with it, see MvMode) on stream s.
+// y = A x (+ the statement MODE fuses with it, see MvMode) on stream s.  T: the dot terms ([2][nz][NQ]).
 template <int NC, int MODE>
-inline void launch_mv(cudaStream_t s, const Geom &g, const double *A, const int32_t *act, const double *xu,
+inline void launch_mv(cudaStream_t s, const Geom &g, const MvMatrix &M, const int32_t *act, const double *xu,
                       const double *xv, double *yu, double *yv, const double *bu, const double *bv, double *ru,
-                      double *rv, const RedCtx &rc) {
+                      double *rv, double *T, const RedCtx &rc) {
     const dim3 grid((unsigned)((g.NQ + kBlock - 1) / kBlock), (unsigned)g.nz);
-    k_mv_nodes<NC, MODE><<<grid, kBlock, 0, s>>>(g, A, act, xu, xv, yu, yv, bu, bv, ru, rv, rc);
+    if (NC == 27 && M.layout == MV_HALF)
+        k_mv_nodes<27, MODE, MV_HALF><<<grid, kBlock, 0, s>>>(g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
+    else if (M.layout == MV_INNER)
+        k_mv_nodes<NC, MODE, MV_INNER><<<grid, kBlock, 0, s>>>(g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
+    else
+        k_mv_nodes<NC, MODE, MV_BOUNDS><<<grid, kBlock, 0, s>>>(g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
 }
 
 // ---------------------------------------------------------------------------

@@ -94,7 +94,7 @@ struct MDesc {
     const int *maps;     // [ntiles][(kTX+2)*(TY+2)] slot maps (k_slot_maps)
     const int *nbrs;     // [ntiles][kNbrStride] tiles owning the tile's live halo columns (k_tile_nbrs)
     int stream;          // matrix loads evict-first (the FP32 matrix exceeds kStreamBytes)
-    int sym;             // 3D, exactly symmetric: A32 and A64i hold the symmetric half (k_to_half)
+    int sym;             // 3D, exactly symmetric: A32 and A64i hold the symmetric half (k_half3d)
     // precond 3, 4: FP32 line factors [u, v][sub, 1/diag, omega, 1/denom][NQ], the lines' right-hand
     // sides rs and solution zs [u, v][NQ]; u planes transposed (column i, row j at i*NY + j) so that
     // the u lines, one per owned row, load and store coalesced
@@ -1757,62 +1757,6 @@ __global__ void k_to_f32(Geom g, const double *__restrict__ src, float4 *__restr
     }
 }
 
-// Exact symmetry of a 3D system, the condition of the symmetric half storage: every lower
-// coupling c < 13 of an owned active row R equals its transpose partner bit for bit -- Auu with
-// Auu, Auv with Avu, Avu with Auv, Avv with Avv -- at the neighbour node n = R + (iA, jA, kA)
-// and the opposite offset 26 - c.  check_symmetry_assembled_matrix_3d, which the reference runs
-// before every 3D solve (glissade_velo_higher.F90:2923-2931), averages such pairs to equality.
-// A difference, or a partner outside the array, sets *flag.  One thread per column.
-__global__ void k_sym_exact3d(Geom g, const int32_t *__restrict__ act, const double *__restrict__ A, int *flag) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= g.NQ) return;
-    const int i = (int)(q % g.NX), j = (int)(q / g.NX);
-    if (!owned(g, i, j) || act[q] == 0) return;
-    const long long plane = (long long)g.nz * g.NQ, bs = 27 * plane;
-    int bad = 0;
-    for (int k = 0; k < g.nz && !bad; ++k)
-        for (int c = 0; c < 13; ++c) {
-            const int iA = c % 3 - 1, jA = (c / 3) % 3 - 1, kA = c / 9 - 1;
-            const int in = i + iA, jn = j + jA, kn = k + kA;
-            if (kn < 0) continue;  // a coupling leaving the column: zero in both layouts
-            if (in < 0 || in >= g.NX || jn < 0 || jn >= g.NY) { bad = 1; break; }
-            const long long e = (long long)c * plane + (long long)k * g.NQ + q;
-            const long long f = (long long)(26 - c) * plane + (long long)kn * g.NQ + (long long)jn * g.NX + in;
-            if (A[e] != A[f] || A[bs + e] != A[2 * bs + f] || A[2 * bs + e] != A[bs + f] ||
-                A[3 * bs + e] != A[3 * bs + f]) {
-                bad = 1;
-                break;
-            }
-        }
-    if (bad) atomicOr(flag, 1);
-}
-
-// The symmetric half copy (3D): the 14 couplings c = 13..26 (the diagonal and the upper
-// offsets) of every node, FP32 as float4 (uu, uv, vu, vv) in planes [c - 13][nz][NQ] and FP64
-// interleaved as {uu, uv}, {vu, vv}; couplings leaving the array are stored as zero, as in
-// k_to_f32.  The kernels read a lower coupling from its transpose partner.
-__global__ void k_to_half(Geom g, const double *__restrict__ src, float4 *__restrict__ dst,
-                          double2 *__restrict__ dst64) {
-    const long long plane = (long long)g.nz * g.NQ;
-    const long long n = 14 * plane;
-    const size_t bs = (size_t)27 * plane;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int h = (int)(e / plane), c = 13 + h;
-        const long long r = e % plane;
-        const int k = (int)(r / g.NQ);
-        const long long q = r % g.NQ;
-        const int i = (int)(q % g.NX), j = (int)(q / g.NX);
-        const int iA = c % 3 - 1, jA = (c / 3) % 3 - 1, kA = c / 9 - 1;
-        const bool in = i + iA >= 0 && i + iA < g.NX && j + jA >= 0 && j + jA < g.NY && k + kA >= 0 && k + kA < g.nz;
-        const size_t f = (size_t)c * plane + r;
-        const double uu = in ? src[f] : 0.0, uv = in ? src[bs + f] : 0.0;
-        const double vu = in ? src[2 * bs + f] : 0.0, vv = in ? src[3 * bs + f] : 0.0;
-        dst[e] = make_float4((float)uu, (float)uv, (float)vu, (float)vv);
-        dst64[2 * e] = make_double2(uu, uv);
-        dst64[2 * e + 1] = make_double2(vu, vv);
-    }
-}
-
 // diag: inverse of the diagonal coefficient (0 where the diagonal is 0), per component
 // sia : Thomas factors of the column tridiagonal (0,0,-1)/(0,0,0)/(0,0,+1) couplings
 template <int NC>
@@ -1875,10 +1819,9 @@ struct MixedBufs {
     int shape_nc = 0;
     int precond = -1;
     float4 *A32 = nullptr;
-    double2 *A64i = nullptr;   // FP64 matrix interleaved per coupling (k_to_f32), or its symmetric half
-    bool sym = false;          // A32 and A64i hold the symmetric half (k_to_half)
-    bool il = false;           // A64i holds the full interleaved FP64 copy (streamed, not symmetric)
-    int *flag = nullptr;       // device word of the symmetry test
+    double2 *A64i = nullptr;   // FP64 matrix interleaved per coupling (k_to_f32)
+    bool sym = false;          // A32 and the Solver's FP64 copy hold the symmetric half (k_half3d)
+    bool il = false;           // A64i holds the full interleaved FP64 copy (3D not symmetric, 2D streamed)
     float *pre = nullptr, *vec = nullptr;
     float *tri = nullptr;      // precond 3, 4: line factors [8][NQ], rs [2][NQ], zs [2][NQ]
     int *maps = nullptr;
@@ -1895,12 +1838,11 @@ struct MixedBufs {
     long long maps_cap = 0;
     void release() {
         for (void *p : {(void *)A32, (void *)A64i, (void *)pre, (void *)vec, (void *)recs, (void *)state, (void *)desc,
-                        (void *)tiles, (void *)ctl, (void *)maps, (void *)nbrs, (void *)bc, (void *)flag, (void *)tri})
+                        (void *)tiles, (void *)ctl, (void *)maps, (void *)nbrs, (void *)bc, (void *)tri})
             if (p) dev_free(p);
         tri = nullptr;
         A32 = nullptr;
         A64i = nullptr;
-        flag = nullptr;
         sym = false;
         il = false;
         pre = vec = nullptr;
