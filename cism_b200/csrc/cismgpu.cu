@@ -1303,16 +1303,15 @@ struct Solver {
             const int global = precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
             double *T = tri.as<double>();
             const long long NQ = g.NQ;
-            const unsigned lb = (tri_lines(g) + kBlock - 1) / kBlock;
             if (NCC == 27) {
-                k_tri_vsum<<<nblocks(NQ), kBlock, 0, stream>>>(g, p.ru, p.rv, T, st);
-                k_tri_lines<<<lb, kBlock, 0, stream>>>(g, global, T + TRS_U * NQ, T + TRS_V * NQ, T + TZS_U * NQ,
-                                                       T + TZS_V * NQ, T, st);
+                k_tri_lines<true><<<tri_blocks(g), kTriThreads, tri_smem(g), stream>>>(
+                    g, global, p.ru, p.rv, T + TZS_U * NQ, T + TZS_V * NQ, T, st);
                 c.zs = T + TZS_U * NQ;
             } else {
                 CU(cudaMemsetAsync(p.zu, 0, NQ * sizeof(double), stream));
                 CU(cudaMemsetAsync(p.zv, 0, NQ * sizeof(double), stream));
-                k_tri_lines<<<lb, kBlock, 0, stream>>>(g, global, p.ru, p.rv, p.zu, p.zv, T, st);
+                k_tri_lines<false><<<tri_blocks(g), kTriThreads, tri_smem(g), stream>>>(g, global, p.ru, p.rv, p.zu,
+                                                                                        p.zv, T, st);
                 halo(p.zu, p.zv);
             }
         }

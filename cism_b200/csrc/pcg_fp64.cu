@@ -997,7 +997,6 @@ __global__ void __launch_bounds__(kBlock) k_sym_check(Geom g, SymIdx L, const in
 enum TriPlane {
     TU_SUB = 0, TU_DG, TU_SP, TU_ADR, TU_OM, TU_DEN,  // u lines: sub, diag, super, 1/diag, omega, 1/denom
     TV_SUB, TV_DG, TV_SP, TV_ADR, TV_OM, TV_DEN,      // v lines
-    TRS_U, TRS_V,                                     // 3D: vertical sums of r
     TZS_U, TZS_V,                                     // 3D: line solution of the summed problem
     NTRI
 };
@@ -1117,93 +1116,149 @@ __global__ void k_tri_factor(Geom g, int global, double *__restrict__ T, SolveSt
     }
 }
 
-// sum(ru(:,i,j)) over levels, in level order (tridiag_solver_local_3d :4585-4590)
-__global__ void k_tri_vsum(Geom g, const double *__restrict__ ru, const double *__restrict__ rv,
-                           double *__restrict__ T, const SolveState *st) {
-    if (st->done) return;
-    const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
-    if (q >= g.NQ) return;
-    double a = 0.0, b = 0.0;
-    for (int k = 0; k < g.nz; ++k) {
-        a = __dadd_rn(a, ru[(long long)k * g.NQ + q]);
-        b = __dadd_rn(b, rv[(long long)k * g.NQ + q]);
-    }
-    T[TRS_U * g.NQ + q] = a;
-    T[TRS_V * g.NQ + q] = b;
-}
-
 // Line solves of tridiag_solver_local_2d (:4985-5013 u, :5041-5069 v) from planes bu, bv into
-// xu, xv, which hold zeros on entry: gamma forward (stored in x), then back substitution.  A
-// line is a chain of dependent operations, so the loads of kTriBatch positions are issued before
-// the chain runs through them (one memory round trip per batch instead of per position); the
-// operations and their order are the reference's.
-constexpr int kTriBatch = 8;
-__global__ void k_tri_lines(Geom g, int global, const double *__restrict__ bu, const double *__restrict__ bv,
-                            double *__restrict__ xu, double *__restrict__ xv, const double *__restrict__ T,
-                            const SolveState *st) {
+// xu, xv, which hold zeros outside the lines: gamma forward, then back substitution.  SUM (3D): the
+// right-hand side is the sum of r over the levels, in level order (tridiag_solver_local_3d :4585-4590).
+// A line is a chain of dependent FP64 operations (three a position forward, two backward), which
+// bounds the launch; so everything else is taken off the chain: a block stages kTriLines lines,
+// kTriChunk positions at a time, in shared memory with all its threads (coalesced for the u lines,
+// whole 32-byte sectors for the v lines, kTriLines adjacent columns), one thread per line runs the
+// recurrences there, and all threads store.  The operations and their order are the reference's.
+// 150x101x11: 22 us for the lines and the level sums; with a thread per line on global memory, all
+// lines in one block, and the sums as a launch of their own, 55 + 6.5.
+constexpr int kTriLines = 4, kTriChunk = 376, kTriThreads = 128;
+static_assert(4 * kTriLines * (kTriChunk + 1) * sizeof(double) <= 48 * 1024, "no opt-in shared memory");
+
+template <bool SUM>
+__global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, const double *__restrict__ bu,
+                                                           const double *__restrict__ bv, double *__restrict__ xu,
+                                                           double *__restrict__ xv, const double *__restrict__ T,
+                                                           const SolveState *st) {
     if (st->done) return;
-    const int t = blockIdx.x * kBlock + threadIdx.x;
-    if (t >= tri_lines(g)) return;
-    bool along_i;
-    int l, s0, s1;
-    tri_line(g, t, along_i, l, s0, s1);
+    extern __shared__ double stri[];  // [b / gamma, sub, 1/denom, omega][line][pitch]
+    const int nu = g.jhi - g.jlo + 1, nug = (nu + kTriLines - 1) / kTriLines;
+    const bool along_i = (int)blockIdx.x < nug;
+    const int l0 = along_i ? g.jlo + (int)blockIdx.x * kTriLines : g.ilo + ((int)blockIdx.x - nug) * kTriLines;
+    const int nl = min(kTriLines, (along_i ? g.jhi : g.ihi) - l0 + 1);
+    const int s0 = along_i ? g.ilo : g.jlo, s1 = along_i ? g.ihi : g.jhi, len = s1 - s0 + 1;
+    const int nch = (len + kTriChunk - 1) / kTriChunk, pitch = min(len, kTriChunk) + 1;
     const double *P = T + (along_i ? TU_SUB : TV_SUB) * g.NQ;
     const double *sub = P, *adr = P + 3 * g.NQ, *om = P + 4 * g.NQ, *den = P + 5 * g.NQ;
     const double *b = along_i ? bu : bv;
     double *x = along_i ? xu : xv;
-    long long e = tri_at(g, along_i, l, s0);
-    double gp = __dmul_rn(b[e], adr[e]);
-    x[e] = gp;
-    for (int s = s0 + 1; s <= s1; s += kTriBatch) {
-        double vb[kTriBatch], vs[kTriBatch], vd[kTriBatch];
+    double *sb = stri, *ss = sb + kTriLines * pitch, *sd = ss + kTriLines * pitch, *so = sd + kTriLines * pitch;
+    const int tid = threadIdx.x;
+    // the elements (line, position) of a chunk: positions run fastest along u lines, lines along v lines
+    auto each = [&](int c0, int n, auto &&f) {
+        for (int w = tid; w < nl * n; w += kTriThreads) {
+            const int ln = along_i ? w / n : w % nl, s = along_i ? w % n : w / nl;
+            f(ln * pitch + s, tri_at(g, along_i, l0 + ln, s0 + c0 + s));
+        }
+    };
+    double gp = 0.0;
+    for (int c = 0; c < nch; ++c) {
+        const int c0 = c * kTriChunk, n = min(kTriChunk, len - c0);
+        each(c0, n, [&](int w, long long e) {
+            double v = 0.0;
+            if (SUM) {
+                for (int k0 = 0; k0 < g.nz; k0 += 8) {
+                    double r[8];
 #pragma unroll
-        for (int u = 0; u < kTriBatch; ++u) {
-            vb[u] = vs[u] = vd[u] = 0.0;
-            if (s + u <= s1) {
-                const long long f = tri_at(g, along_i, l, s + u);
-                vb[u] = b[f];
-                vs[u] = sub[f];
-                vd[u] = den[f];
+                    for (int u = 0; u < 8; ++u) r[u] = (k0 + u < g.nz) ? b[(long long)(k0 + u) * g.NQ + e] : 0.0;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (k0 + u < g.nz) v = __dadd_rn(v, r[u]);
+                }
+            } else {
+                v = b[e];
+            }
+            sb[w] = v;
+            ss[w] = sub[e];
+            sd[w] = den[e];
+            if (nch == 1) so[w] = om[e];
+        });
+        __syncthreads();
+        if (tid < nl) {
+            double *vb = sb + tid * pitch;
+            const double *vs = ss + tid * pitch, *vd = sd + tid * pitch;
+            int s = 0;
+            if (c == 0) {
+                gp = __dmul_rn(vb[0], adr[tri_at(g, along_i, l0 + tid, s0)]);
+                vb[0] = gp;
+                s = 1;
+            }
+            for (; s < n; s += 8) {
+                double r[8], p[8], d[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int w = min(s + u, n - 1);
+                    r[u] = vb[w];
+                    p[u] = vs[w];
+                    d[u] = vd[w];
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (s + u < n) {
+                        gp = __dmul_rn(__dsub_rn(r[u], __dmul_rn(p[u], gp)), d[u]);
+                        vb[s + u] = gp;
+                    }
             }
         }
-#pragma unroll
-        for (int u = 0; u < kTriBatch; ++u)
-            if (s + u <= s1) {
-                gp = __dmul_rn(__dsub_rn(vb[u], __dmul_rn(vs[u], gp)), vd[u]);
-                x[tri_at(g, along_i, l, s + u)] = gp;
-            }
+        __syncthreads();
+        if (nch > 1) {
+            each(c0, n, [&](int w, long long e) { x[e] = sb[w]; });
+            __syncthreads();
+        }
     }
     double xn = gp;
-    for (int s = s1 - 1; s >= s0; s -= kTriBatch) {
-        double vx[kTriBatch], vo[kTriBatch];
-#pragma unroll
-        for (int u = 0; u < kTriBatch; ++u) {
-            vx[u] = vo[u] = 0.0;
-            if (s - u >= s0) {
-                const long long f = tri_at(g, along_i, l, s - u);
-                vx[u] = x[f];  // this thread's forward value
-                vo[u] = om[f];
-            }
+    for (int c = nch - 1; c >= 0; --c) {
+        const int c0 = c * kTriChunk, n = min(kTriChunk, len - c0);
+        if (nch > 1) {
+            each(c0, n, [&](int w, long long e) {
+                sb[w] = x[e];  // gamma, as this block stored it
+                so[w] = om[e];
+            });
+            __syncthreads();
         }
+        if (tid < nl) {
+            double *vb = sb + tid * pitch;
+            const double *vo = so + tid * pitch;
+            for (int s = (c == nch - 1) ? n - 2 : n - 1; s >= 0; s -= 8) {
+                double r[8], o[8];
 #pragma unroll
-        for (int u = 0; u < kTriBatch; ++u)
-            if (s - u >= s0) {
-                xn = __dsub_rn(vx[u], __dmul_rn(vo[u], xn));
-                x[tri_at(g, along_i, l, s - u)] = xn;
-            }
-    }
-    if (!global)
-        for (int s = s0 - 1; s >= 0; s -= kTriBatch) {
-            double vo[kTriBatch];
-#pragma unroll
-            for (int u = 0; u < kTriBatch; ++u) vo[u] = (s - u >= 0) ? om[tri_at(g, along_i, l, s - u)] : 0.0;
-#pragma unroll
-            for (int u = 0; u < kTriBatch; ++u)
-                if (s - u >= 0) {
-                    xn = __dsub_rn(0.0, __dmul_rn(vo[u], xn));
-                    x[tri_at(g, along_i, l, s - u)] = xn;
+                for (int u = 0; u < 8; ++u) {
+                    const int w = max(s - u, 0);
+                    r[u] = vb[w];
+                    o[u] = vo[w];
                 }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (s - u >= 0) {
+                        xn = __dsub_rn(r[u], __dmul_rn(o[u], xn));
+                        vb[s - u] = xn;
+                    }
+            }
         }
+        __syncthreads();
+        each(c0, n, [&](int w, long long e) { x[e] = sb[w]; });
+        __syncthreads();
+    }
+    // the local back substitution runs on below the owned range (:4999-5001; gamma is zero there)
+    if (!global && tid < nl)
+        for (int s = s0 - 1; s >= 0; --s) {
+            const long long e = tri_at(g, along_i, l0 + tid, s);
+            xn = __dsub_rn(0.0, __dmul_rn(om[e], xn));
+            x[e] = xn;
+        }
+}
+
+// Blocks and shared memory of k_tri_lines.
+inline unsigned tri_blocks(const Geom &g) {
+    return (unsigned)((g.jhi - g.jlo + kTriLines) / kTriLines + (g.ihi - g.ilo + kTriLines) / kTriLines);
+}
+inline size_t tri_smem(const Geom &g) {
+    const int len = g.ihi - g.ilo > g.jhi - g.jlo ? g.ihi - g.ilo + 1 : g.jhi - g.jlo + 1;
+    return (size_t)4 * kTriLines * ((len < kTriChunk ? len : kTriChunk) + 1) * sizeof(double);
 }
 
 // ---------------------------------------------------------------------------
