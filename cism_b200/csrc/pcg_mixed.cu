@@ -381,18 +381,16 @@ __device__ __forceinline__ double ld_stream(const double *p, unsigned long long 
     asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
     return v;
 }
-__device__ __forceinline__ double2 ld_stream(const double2 *p, unsigned long long pol) {
-    double2 v;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-        : "=d"(v.x), "=d"(v.y)
+
+// The FP64 coefficients of one coupling and node, (uu, uv, vu, vv), in one 32-byte load (as two
+// 16-byte loads each warp fetched every sector twice: 6 sliding systems of 64..256 columns 476 -> 452 ms).
+__device__ __forceinline__ Dbl4 ld_coupling(const double2 *p, unsigned long long pol) {
+    Dbl4 v;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f64 {%0, %1, %2, %3}, [%4], %5;"
+        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
         : "l"(p), "l"(pol));
     return v;
 }
-
-// Loads of the symmetric half copy: every stored coupling is read twice in a step, by its
-// node and by its transpose partner's node, close together in time.
-__device__ __forceinline__ float4 ld_half(const float4 *p, unsigned long long pol) { return ld_stream(p, pol); }
-__device__ __forceinline__ double2 ld_half(const double2 *p, unsigned long long pol) { return ld_stream(p, pol); }
 
 // Loads of data that other CTAs wrote earlier in the same launch go through L2
 // (ld.global.cg): L1 is not coherent across SMs.
@@ -611,28 +609,25 @@ __device__ __forceinline__ void residual_pass(const MDesc &D, const int *smap, i
                                 x2 = fma(alpha64, (double)sdn[(nz + k + kA) * NS + sn], x2);
                             }
                             if (HALF) {
-                                double2 au, av;
+                                Dbl4 a4;
                                 if (c >= 13) {
-                                    const size_t h = (size_t)(c - 13) * plane + e;
-                                    au = ld_half(A2 + 2 * h, pol);
-                                    av = ld_half(A2 + 2 * h + 1, pol);
+                                    a4 = ld_coupling(A2 + 2 * ((size_t)(c - 13) * plane + e), pol);
                                 } else {  // partner n = (k+kA, i+iA, j+jA), coupling 26 - c, blocks swapped
                                     const size_t h = (size_t)(13 - c) * plane + (size_t)(k + kA) * NQ +
                                                      (size_t)((j + jA) * g.NX + (i + iA));
-                                    const double2 pu = ld_half(A2 + 2 * h, pol), pv = ld_half(A2 + 2 * h + 1, pol);
-                                    au = make_double2(pu.x, pv.x);  // uu, uv(R) = vu(n)
-                                    av = make_double2(pu.y, pv.y);  // vu(R) = uv(n), vv
+                                    const Dbl4 pa = ld_coupling(A2 + 2 * h, pol);
+                                    a4 = Dbl4{pa.x, pa.z, pa.y, pa.w};  // uv(R) = vu(n), vu(R) = uv(n)
                                 }
-                                yu[u] = fma(au.x, x1, yu[u]);
-                                yu[u] = fma(au.y, x2, yu[u]);
-                                yv[u] = fma(av.x, x1, yv[u]);
-                                yv[u] = fma(av.y, x2, yv[u]);
+                                yu[u] = fma(a4.x, x1, yu[u]);
+                                yu[u] = fma(a4.y, x2, yu[u]);
+                                yv[u] = fma(a4.z, x1, yv[u]);
+                                yv[u] = fma(a4.w, x2, yv[u]);
                             } else if (IL) {
-                                const double2 au = ld_stream(A2 + 2 * a, pol), av = ld_stream(A2 + 2 * a + 1, pol);
-                                yu[u] = fma(au.x, x1, yu[u]);
-                                yu[u] = fma(au.y, x2, yu[u]);
-                                yv[u] = fma(av.x, x1, yv[u]);
-                                yv[u] = fma(av.y, x2, yv[u]);
+                                const Dbl4 a4 = ld_coupling(A2 + 2 * a, pol);
+                                yu[u] = fma(a4.x, x1, yu[u]);
+                                yu[u] = fma(a4.y, x2, yu[u]);
+                                yv[u] = fma(a4.z, x1, yv[u]);
+                                yv[u] = fma(a4.w, x2, yv[u]);
                             } else {
                                 yu[u] = fma(ld_stream(Auu + a, pol), x1, yu[u]);
                                 yu[u] = fma(ld_stream(Auv + a, pol), x2, yu[u]);
@@ -708,27 +703,22 @@ __device__ __forceinline__ void residual_tile(const MDesc &D, const int *smap, i
                             const int iA = c % 3 - 1, jA = (c / 3) % 3 - 1, kA = c / 9 - 1;
                             const int zi = (k + 1 + kA) * NS + s + iA + (kTX + 2) * jA;
                             const double x1 = sxu[zi], x2 = sxv[zi];
-                            double2 au, av;
+                            Dbl4 a4;
                             if (!HALF) {
-                                const size_t h = (size_t)c * plane + e;
-                                au = ld_stream(A2 + 2 * h, pol);
-                                av = ld_stream(A2 + 2 * h + 1, pol);
+                                a4 = ld_coupling(A2 + 2 * ((size_t)c * plane + e), pol);
                             } else if (c >= 13) {
-                                const size_t h = (size_t)(c - 13) * plane + e;
-                                au = ld_half(A2 + 2 * h, pol);
-                                av = ld_half(A2 + 2 * h + 1, pol);
+                                a4 = ld_coupling(A2 + 2 * ((size_t)(c - 13) * plane + e), pol);
                             } else {  // partner n = (k+kA, i+iA, j+jA), coupling 26 - c, blocks swapped
                                 const int kk = k + kA < 0 ? 0 : k + kA;  // level -1: its x row is zero
                                 const size_t h = (size_t)(13 - c) * plane + (size_t)kk * NQ +
                                                  (size_t)((j + jA) * g.NX + (i + iA));
-                                const double2 pu = ld_half(A2 + 2 * h, pol), pv = ld_half(A2 + 2 * h + 1, pol);
-                                au = make_double2(pu.x, pv.x);
-                                av = make_double2(pu.y, pv.y);
+                                const Dbl4 pa = ld_coupling(A2 + 2 * h, pol);
+                                a4 = Dbl4{pa.x, pa.z, pa.y, pa.w};
                             }
-                            yu[u] = fma(au.x, x1, yu[u]);
-                            yu[u] = fma(au.y, x2, yu[u]);
-                            yv[u] = fma(av.x, x1, yv[u]);
-                            yv[u] = fma(av.y, x2, yv[u]);
+                            yu[u] = fma(a4.x, x1, yu[u]);
+                            yu[u] = fma(a4.y, x2, yu[u]);
+                            yv[u] = fma(a4.z, x1, yv[u]);
+                            yv[u] = fma(a4.w, x2, yv[u]);
                         }
                     }
                 }
@@ -1248,10 +1238,10 @@ __device__ void tile_step(const MState &S, int tile, bool resident, int TYmax, M
                                         const float z1 = szu[zi], z2 = szv[zi];
                                         float4 a;
                                         if (c >= 13) {
-                                            a = ld_half(A4 + (size_t)(c - 13) * plane + e, pol);
+                                            a = ld_stream(A4 + (size_t)(c - 13) * plane + e, pol);
                                         } else {
                                             const int kk = k + kA < 0 ? 0 : k + kA;
-                                            const float4 pa = ld_half(A4 + (size_t)(13 - c) * plane + kk * NQ +
+                                            const float4 pa = ld_stream(A4 + (size_t)(13 - c) * plane + kk * NQ +
                                                                             (j + jA) * g.NX + (i + iA), pol);
                                             a = make_float4(pa.x, pa.z, pa.y, pa.w);
                                         }
