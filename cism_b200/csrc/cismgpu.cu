@@ -1813,8 +1813,9 @@ static MDesc mixed_desc(const Solver &sv, int precond, int TY) {  // TY: the sol
     return D;
 }
 
-// Shared memory of the mixed kernel for a tile height (resident: 2D launches with one tile
-// per CTA keep the tile's FP32 matrix in shared memory).
+// Shared memory of the mixed kernel that tile heights are planned with (resident: 2D launches with
+// one tile per CTA keep the tile's FP32 matrix in shared memory).  A launch takes what its level count
+// needs, mixed_smem_of.
 static size_t mixed_smem(bool is3d, int nzm, int TY, bool resident = false) {
     if (!is3d) return MLayout<9, 1>(TY, resident).bytes();
     if (nzm == 16) return MLayout<27, 16>(TY, false).bytes();
@@ -2065,50 +2066,42 @@ static int mixed_reset(Solver &sv, cudaStream_t s) {
     return CISMGPU_OK;
 }
 
-// Co-resident grid of a launch (sets the kernel's shared-memory attribute; call outside any
-// stream capture).  0 if the kernel does not fit.
-static int mixed_launch_grid(bool is3d, int nzm, int TY, bool resident, int ntiles) {
-    const int grid = mixed_grid(is3d, nzm, TY, resident);
-    if (grid < 1) return 0;
-    if (resident && grid < ntiles) return 0;
-    return std::min(grid, ntiles);
+// Shared memory of a launch of solves of up to nzl levels and tile height TY.
+static size_t mixed_smem_of(bool is3d, int nzm, int TY, bool resident, int nzl) {
+    if (!is3d) return MLayout<9, 1>(TY, resident).bytes();
+    if (nzm == 16) return MLayout<27, 16>(TY, false, nzl).bytes();
+    return MLayout<27, 32>(TY, false, nzl).bytes();
+}
+
+// Co-resident grid of a launch of kernel k and its shared memory (sets the kernel's shared-memory
+// attribute; call outside any stream capture).  grid 0: the kernel does not fit.
+struct MPlan {
+    int grid = 0, nzl = 1;
+    size_t smem = 0;
+};
+static MPlan mixed_plan(const void *k, bool is3d, int nzm, int TY, bool resident, int nzl, size_t least = 0) {
+    MPlan P;
+    P.nzl = is3d ? nzl : 1;
+    P.smem = std::max(least, mixed_smem_of(is3d, nzm, TY, resident, P.nzl));
+    P.grid = smem_grid(k, P.smem);
+    return P;
+}
+
+// The plan of a single-solve launch (k_mixed): at most one CTA per tile; resident: exactly one.
+static MPlan mixed_launch_plan(const Solver &sv, int nzm, int TY, bool resident, int ntiles) {
+    MPlan P = mixed_plan(mixed_kernel(sv.is3d, nzm), sv.is3d, nzm, TY, resident, sv.g.nz);
+    if (resident && P.grid < ntiles) P.grid = 0;
+    P.grid = std::min(P.grid, ntiles);
+    return P;
 }
 
 template <int NC, int NZM>
 static int mixed_launch(const MDesc *d_descs, MState *d_states, const MTile *d_tiles, int ntiles, int TY,
-                        int resident, MCtl *d_ctl, int max_steps, int grid, cudaStream_t s) {
-    const size_t smem = MLayout<NC, NZM>(TY, resident != 0).bytes();
+                        int resident, MCtl *d_ctl, int max_steps, const MPlan &P, cudaStream_t s) {
+    int nzl = P.nzl;
     void *args[] = {(void *)&d_descs, (void *)&d_states, (void *)&d_tiles, (void *)&ntiles, (void *)&TY,
-                    (void *)&resident, (void *)&d_ctl, (void *)&max_steps};
-    CU(cudaLaunchCooperativeKernel((const void *)k_mixed<NC, NZM>, dim3(grid), dim3(kBlock), args, smem, s));
-    return CISMGPU_OK;
-}
-
-template <int NC, int NZM>
-static int mixed_dyn_launch(const MDesc *d_descs, MState *const *d_states, const unsigned *d_tick0, int nsolve,
-                            const MTile *d_tiles, int ntiles, int TY, MCtl *d_ctl, int max_steps, int grid,
-                            cudaStream_t s) {
-    const size_t smem = MLayout<NC, NZM>(TY, false).bytes();
-    int TY2 = TY;
-    void *args[] = {(void *)&d_descs, (void *)&d_states, (void *)&d_tick0, (void *)&nsolve, (void *)&d_tiles,
-                    (void *)&ntiles, (void *)&TY, (void *)&TY2, (void *)&d_ctl, (void *)&max_steps};
-    CU(cudaLaunchCooperativeKernel((const void *)k_mixed_dyn<NC, NZM>, dim3(grid), dim3(kBlock), args, smem, s));
-    return CISMGPU_OK;
-}
-
-// Shared memory of the 2D + 3D (nz <= 16) dynamic kernel: the larger of the two layouts.
-static size_t mixed_multi_smem(int TY3, int TY2) {
-    return std::max(MLayout<27, 16>(TY3, false).bytes(), MLayout<9, 1>(TY2, false).bytes());
-}
-
-// One launch of 2D and 3D (nz <= 16) solves together: 3D tiles of height at most TY3, 2D at most TY2.
-static int mixed_multi_launch(const MDesc *d_descs, MState *const *d_states, const unsigned *d_tick0, int nsolve,
-                              const MTile *d_tiles, int ntiles, int TY3, int TY2, MCtl *d_ctl, int max_steps,
-                              int grid, cudaStream_t s) {
-    const size_t smem = mixed_multi_smem(TY3, TY2);
-    void *args[] = {(void *)&d_descs, (void *)&d_states, (void *)&d_tick0, (void *)&nsolve, (void *)&d_tiles,
-                    (void *)&ntiles, (void *)&TY3, (void *)&TY2, (void *)&d_ctl, (void *)&max_steps};
-    CU(cudaLaunchCooperativeKernel((const void *)k_mixed_dyn<27, 16, true>, dim3(grid), dim3(kBlock), args, smem, s));
+                    (void *)&resident, (void *)&nzl, (void *)&d_ctl, (void *)&max_steps};
+    CU(cudaLaunchCooperativeKernel((const void *)k_mixed<NC, NZM>, dim3(P.grid), dim3(kBlock), args, P.smem, s));
     return CISMGPU_OK;
 }
 
@@ -2118,28 +2111,31 @@ static const void *mixed_dyn_kernel(bool is3d, int nzm) {
     return (const void *)k_mixed_dyn<27, 32>;
 }
 
-static int mixed_multi_grid(int TY3, int TY2) {
-    return smem_grid((const void *)k_mixed_dyn<27, 16, true>, mixed_multi_smem(TY3, TY2));
+// The plan of a dynamic launch of one class; of 2D and 3D (nz <= 16) solves together (TY2 > 0), whose
+// shared memory is the larger of the two layouts: 3D tiles of height at most TY, 2D at most TY2.
+static MPlan mixed_dyn_plan(bool is3d, int nzm, int TY, int TY2, int nzl) {
+    if (TY2 > 0)
+        return mixed_plan((const void *)k_mixed_dyn<27, 16, true>, true, 16, TY, false, nzl,
+                          MLayout<9, 1>(TY2, false).bytes());
+    return mixed_plan(mixed_dyn_kernel(is3d, nzm), is3d, nzm, TY, false, nzl);
 }
 
-// Co-resident CTAs of the dynamic kernel at tile height TY (0 if it does not fit).
-static int mixed_dyn_grid(bool is3d, int nzm, int TY) {
-    return smem_grid(mixed_dyn_kernel(is3d, nzm), mixed_smem(is3d, nzm, TY, false));
-}
-
-static int mixed_dyn_dispatch(bool is3d, int nzm, const MDesc *d, MState *const *st, const unsigned *tick0, int nsolve,
-                              const MTile *t, int nt, int TY, MCtl *ctl, int max_steps, int grid, cudaStream_t s) {
-    if (!is3d) return mixed_dyn_launch<9, 1>(d, st, tick0, nsolve, t, nt, TY, ctl, max_steps, grid, s);
-    if (nzm == 16) return mixed_dyn_launch<27, 16>(d, st, tick0, nsolve, t, nt, TY, ctl, max_steps, grid, s);
-    return mixed_dyn_launch<27, 32>(d, st, tick0, nsolve, t, nt, TY, ctl, max_steps, grid, s);
+static int mixed_dyn_launch(bool is3d, int nzm, const MDesc *d_descs, MState *const *d_states, const unsigned *d_tick0,
+                            int nsolve, const MTile *d_tiles, int ntiles, int TY, int TY2, MCtl *d_ctl, int max_steps,
+                            const MPlan &P, cudaStream_t s) {
+    const void *k = TY2 > 0 ? (const void *)k_mixed_dyn<27, 16, true> : mixed_dyn_kernel(is3d, nzm);
+    int nzl = P.nzl, ty2 = TY2 > 0 ? TY2 : TY;
+    void *args[] = {(void *)&d_descs, (void *)&d_states, (void *)&d_tick0, (void *)&nsolve, (void *)&d_tiles,
+                    (void *)&ntiles, (void *)&TY, (void *)&ty2, (void *)&nzl, (void *)&d_ctl, (void *)&max_steps};
+    CU(cudaLaunchCooperativeKernel(k, dim3(P.grid), dim3(kBlock), args, P.smem, s));
+    return CISMGPU_OK;
 }
 
 static int mixed_dispatch(bool is3d, int nzm, const MDesc *d, MState *st, const MTile *t, int nt, int TY,
-                          bool resident, MCtl *ctl, int max_steps, int grid, cudaStream_t s) {
-    const int res = resident ? 1 : 0;
-    if (!is3d) return mixed_launch<9, 1>(d, st, t, nt, TY, res, ctl, max_steps, grid, s);
-    if (nzm == 16) return mixed_launch<27, 16>(d, st, t, nt, TY, 0, ctl, max_steps, grid, s);
-    return mixed_launch<27, 32>(d, st, t, nt, TY, 0, ctl, max_steps, grid, s);
+                          bool resident, MCtl *ctl, int max_steps, const MPlan &P, cudaStream_t s) {
+    if (!is3d) return mixed_launch<9, 1>(d, st, t, nt, TY, resident ? 1 : 0, ctl, max_steps, P, s);
+    if (nzm == 16) return mixed_launch<27, 16>(d, st, t, nt, TY, 0, ctl, max_steps, P, s);
+    return mixed_launch<27, 32>(d, st, t, nt, TY, 0, ctl, max_steps, P, s);
 }
 
 static double mixed_iter_bytes(const Solver &sv, int precond) {
@@ -2176,9 +2172,9 @@ static int mixed_run(Solver &sv, int precond, int ncheck, double tol, int maxite
         CU(cudaEventCreate(&e1));
         CU(cudaEventRecord(e0, stream));
     }
-    const int grid = mixed_launch_grid(is3d, nzm, TY, resident, m.ntiles);
-    if (grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
-    TRY(mixed_dispatch(is3d, nzm, m.desc, m.state, m.tiles, m.ntiles, TY, resident, m.ctl, max_steps, grid, stream));
+    const MPlan P = mixed_launch_plan(sv, nzm, TY, resident, m.ntiles);
+    if (P.grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
+    TRY(mixed_dispatch(is3d, nzm, m.desc, m.state, m.tiles, m.ntiles, TY, resident, m.ctl, max_steps, P, stream));
     if (ms) CU(cudaEventRecord(e1, stream));
     k_mstate_to_solve<<<1, 1, 0, stream>>>(m.state, sv.state.as<SolveState>(), m.ctl);
     CU(cudaGetLastError());
@@ -2691,7 +2687,8 @@ static int oneshot_global_sum(int nx, int ny, int nz, const cismgpu_par_t *par, 
 struct MixedBatch {
     std::vector<Solver *> svs;
     bool is3d = false;
-    int nzm = 0, TYmax = 1, grid = 0, ntl = 0, max_steps = 0;
+    int nzm = 0, TYmax = 1, ntl = 0, max_steps = 0;
+    MPlan plan;
     void *dmem = nullptr;
     MDesc *d_descs = nullptr;
     MState *d_states = nullptr, *d_states0 = nullptr;
@@ -2733,9 +2730,11 @@ static int batch_prepare(MixedBatch &B, int precond, int ncheck, double tol, int
         for (int k = 0; k < tiles_for(sv.g, tys[t]); ++k) tl.push_back(MTile{t, k});
     }
     for (int t = 0; t < n; ++t) CU(cudaStreamSynchronize(B.svs[t]->stream));
-    B.grid = mixed_dyn_grid(B.is3d, B.nzm, B.TYmax);
-    if (B.grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
-    if ((long long)n > (long long)B.grid * kMaxCtaSolves)
+    int nzl = 1;
+    for (const Solver *sv : B.svs) nzl = std::max(nzl, sv->g.nz);
+    B.plan = mixed_dyn_plan(B.is3d, B.nzm, B.TYmax, 0, nzl);
+    if (B.plan.grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
+    if ((long long)n > (long long)B.plan.grid * kMaxCtaSolves)
         return fail(CISMGPU_EUNSUPPORTED, "too many systems for one launch");
     B.ntl = (int)tl.size();
     B.max_steps = 4 * maxiters + 16;
@@ -2789,8 +2788,8 @@ static int batch_enqueue(MixedBatch &B, cudaStream_t s) {
     for (Solver *sv : B.svs) TRY(mixed_reset(*sv, s));
     CU(cudaMemcpyAsync(B.d_states, B.d_states0, n * sizeof(MState), cudaMemcpyDeviceToDevice, s));
     CU(cudaMemcpyAsync(B.d_ctl, B.d_ctl0, sizeof(MCtl), cudaMemcpyDeviceToDevice, s));
-    TRY(mixed_dyn_dispatch(B.is3d, B.nzm, B.d_descs, B.d_sptr, B.d_tick0, n, B.d_tiles, B.ntl, B.TYmax, B.d_ctl,
-                           B.max_steps, B.grid, s));
+    TRY(mixed_dyn_launch(B.is3d, B.nzm, B.d_descs, B.d_sptr, B.d_tick0, n, B.d_tiles, B.ntl, B.TYmax, 0, B.d_ctl,
+                         B.max_steps, B.plan, s));
     k_mstates_to_solves<<<(n + 127) / 128, 128, 0, s>>>(B.d_states, B.d_dst, n, B.d_ctl);
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(B.h_states, B.d_states, n * sizeof(MState), cudaMemcpyDeviceToHost, s));

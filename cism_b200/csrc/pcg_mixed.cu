@@ -333,24 +333,25 @@ struct MHead {
     MTile tl[kTilesCached];    // the first kTilesCached of them
 };
 
-// Dynamic shared memory: head | map[NS] | z[2][KP][NS] | rt[2][NZM][NT]
-//                        | (resident launches) A[4][NC][NZM*NT] FP32 matrix of the CTA's tile
-// sized for the launch's largest tile height.
+// Dynamic shared memory: head | map[NS] | z[2][KP][NS] | rt[2][nz][NT]
+//                        | (resident launches) A[4][NC][nz*NT] FP32 matrix of the CTA's tile
+// sized for the launch's largest tile height and level count nzl (a solve's own arrays use its own
+// strides; what it does not take stays L1).  Tile heights are planned with nzl = NZM.
 template <int NC, int NZM>
 struct MLayout {
-    static constexpr int KP = (NC == 27) ? NZM + 2 : 1;  // z levels with a zero row above and below
-    int NS, NT;
+    int NS, NT, nzl, KP;  // KP: z levels with a zero row above and below
     bool resA;
-    __host__ __device__ MLayout(int TY, bool resident) : NS((kTX + 2) * (TY + 2)), NT(kTX * TY), resA(resident) {}
+    __host__ __device__ MLayout(int TY, bool resident, int levels = NZM)
+        : NS((kTX + 2) * (TY + 2)), NT(kTX * TY), nzl(levels), KP((NC == 27) ? levels + 2 : 1), resA(resident) {}
     __host__ __device__ size_t off_map() const { return (sizeof(MHead) + 15) / 16 * 16; }
     __host__ __device__ size_t off_z() const { return (off_map() + 4 * (size_t)NS + 15) / 16 * 16; }
     __host__ __device__ size_t off_rt() const { return off_z() + 4 * (size_t)2 * KP * NS; }
-    __host__ __device__ size_t off_A() const { return (off_rt() + 4 * (size_t)2 * NZM * NT + 15) / 16 * 16; }
+    __host__ __device__ size_t off_A() const { return (off_rt() + 4 * (size_t)2 * nzl * NT + 15) / 16 * 16; }
     // 3D FP64 check steps (up to 16 levels): x (updated by the step's d) of the tile and its halo
     // ring, all levels with a zero row above and below, [2][KP][NS] doubles over the z and rt regions
     __host__ __device__ size_t off_x64() const { return off_z(); }
     __host__ __device__ size_t bytes() const {
-        size_t b = off_A() + (resA ? 4 * (size_t)4 * NC * NZM * NT : 0);
+        size_t b = off_A() + (resA ? 4 * (size_t)4 * NC * nzl * NT : 0);
         if (NC == 27 && NZM <= 16) {  // (32 levels keep the per-coupling residual_pass: the tile
                                       // would halve their occupancy)
             const size_t bx = off_x64() + 8 * (size_t)2 * KP * NS;
@@ -473,69 +474,63 @@ __global__ void k_tile_nbrs(MDesc D, const int *maps, int *nbrs) {
     for (int k = 0; k < n; ++k) out[1 + k] = list[k];
 }
 
-// z = M^-1 r on one column of the SIA tridiagonal, in place in smem (zc = z[c][0][0],
-// row stride NS; level k at row k+1), FP32.  The column's factors are loaded in one
-// batch first: a load inside the recurrence would cost a memory round trip per level.
+// z = M^-1 r on one component of one column of the SIA tridiagonal, FP32, in place in smem (z[k * NS]
+// is level k).  f: the factors 1/beta, sb and gamma of the column in HBM ([3][nz][NQ]), loaded in one
+// batch first: a load inside the recurrence would cost a memory round trip per level.  The address and
+// the strides are opaque to the compiler, which otherwise carries the 3 NZM offsets through the whole
+// step and spills for it (16 levels: 440 -> 425 ms on a 6-member batch; 21 levels: 1.73 -> 1.57 ms).
 template <int NZM>
-__device__ __forceinline__ void sia_col(const MDesc &D, float *zc, int NS, int s, int q, int c0, int c1) {
-    const int nz = D.g.nz;
-    const int NQ = (int)D.g.NQ;
-    const int plane = nz * NQ;
-    constexpr int KP = NZM + 2;
-    for (int c = c0; c <= c1; ++c) {
-        float *z = zc + c * KP * NS + NS + s;  // z[k * NS] is level k
-        const float *ib = D.pre + (c * 3 + 0) * plane, *sb = D.pre + (c * 3 + 1) * plane,
-                    *gm = D.pre + (c * 3 + 2) * plane;
-        float fib[NZM], fsb[NZM], fgm[NZM];
+__device__ __forceinline__ void sia_col(int nz, float *z, int NS, const float *f, int plane, int NQ) {
+    asm volatile("" : "+l"(f), "+r"(plane), "+r"(NQ));
+    float fib[NZM], fsb[NZM], fgm[NZM];
 #pragma unroll
-        for (int k = 0; k < NZM; ++k) {
-            const bool in = k < nz;
-            fib[k] = in ? __ldg(ib + k * NQ + q) : 0.0f;
-            fsb[k] = in ? __ldg(sb + k * NQ + q) : 0.0f;
-            fgm[k] = in ? __ldg(gm + k * NQ + q) : 0.0f;
-        }
-        // forward: y_1 = r_1/beta_1; y_k = (r_k - sb_k y_{k-1})/beta_k; back: z_k = y_k - gamma_{k+1} z_{k+1}
-        if (NZM <= 16) {
-            // the column in registers: its shared-memory loads issue together, and the recurrences
-            // wait on arithmetic alone (the same operations in the same order as below)
-            float zz[NZM];
+    for (int k = 0; k < NZM; ++k) {
+        const bool in = k < nz;
+        fib[k] = in ? f[k * NQ] : 0.0f;
+        fsb[k] = (in && k > 0) ? f[plane + k * NQ] : 0.0f;
+        fgm[k] = (in && k > 0) ? f[2 * plane + k * NQ] : 0.0f;
+    }
+    // forward: y_1 = r_1/beta_1; y_k = (r_k - sb_k y_{k-1})/beta_k; back: z_k = y_k - gamma_{k+1} z_{k+1}
+    if (NZM <= 16) {
+        // the column in registers: its shared-memory loads issue together, and the recurrences
+        // wait on arithmetic alone (the same operations in the same order as below)
+        float zz[NZM];
 #pragma unroll
-            for (int k = 0; k < NZM; ++k) zz[k] = (k < nz) ? z[k * NS] : 0.0f;
-            float prev = zz[0] * fib[0];
-            zz[0] = prev;
+        for (int k = 0; k < NZM; ++k) zz[k] = (k < nz) ? z[k * NS] : 0.0f;
+        float prev = zz[0] * fib[0];
+        zz[0] = prev;
 #pragma unroll
-            for (int k = 1; k < NZM; ++k)
-                if (k < nz) {
-                    prev = (zz[k] - fsb[k] * prev) * fib[k];
-                    zz[k] = prev;
-                }
-            float next = prev;
+        for (int k = 1; k < NZM; ++k)
+            if (k < nz) {
+                prev = (zz[k] - fsb[k] * prev) * fib[k];
+                zz[k] = prev;
+            }
+        float next = prev;
 #pragma unroll
-            for (int k = NZM - 2; k >= 0; --k)
-                if (k < nz - 1) {
-                    next = zz[k] - fgm[k + 1] * next;
-                    zz[k] = next;
-                }
+        for (int k = NZM - 2; k >= 0; --k)
+            if (k < nz - 1) {
+                next = zz[k] - fgm[k + 1] * next;
+                zz[k] = next;
+            }
 #pragma unroll
-            for (int k = 0; k < NZM; ++k)
-                if (k < nz) z[k * NS] = zz[k];
-        } else {
-            float prev = z[0] * fib[0];
-            z[0] = prev;
+        for (int k = 0; k < NZM; ++k)
+            if (k < nz) z[k * NS] = zz[k];
+    } else {
+        float prev = z[0] * fib[0];
+        z[0] = prev;
 #pragma unroll
-            for (int k = 1; k < NZM; ++k)
-                if (k < nz) {
-                    prev = (z[k * NS] - fsb[k] * prev) * fib[k];
-                    z[k * NS] = prev;
-                }
-            float next = prev;
+        for (int k = 1; k < NZM; ++k)
+            if (k < nz) {
+                prev = (z[k * NS] - fsb[k] * prev) * fib[k];
+                z[k * NS] = prev;
+            }
+        float next = prev;
 #pragma unroll
-            for (int k = NZM - 2; k >= 0; --k)
-                if (k < nz - 1) {
-                    next = z[k * NS] - fgm[k + 1] * next;
-                    z[k * NS] = next;
-                }
-        }
+        for (int k = NZM - 2; k >= 0; --k)
+            if (k < nz - 1) {
+                next = z[k * NS] - fgm[k + 1] * next;
+                z[k * NS] = next;
+            }
     }
 }
 
@@ -661,9 +656,8 @@ __device__ __forceinline__ void residual_pass(const MDesc &D, const int *smap, i
 template <int NZM, bool HALF>
 __device__ __forceinline__ void residual_tile(const MDesc &D, const int *smap, int TY, int i0, int j0, int rpar,
                                               const double *sx, double &p0, double &p1) {
-    constexpr int KP = NZM + 2;
     const Geom &g = D.g;
-    const int nz = g.nz;
+    const int nz = g.nz, KP = nz + 2;
     const int NQ = (int)g.NQ;
     const int plane = nz * NQ;
     const int NT = kTX * TY;
@@ -743,9 +737,8 @@ __device__ __forceinline__ void residual_tile(const MDesc &D, const int *smap, i
 template <int NZM>
 __device__ __forceinline__ void fill_x_tile(const MDesc &D, const int *smap, int TY, int par, bool upd, float beta,
                                             double alpha64, double *sx) {
-    constexpr int KP = NZM + 2;
     const Geom &g = D.g;
-    const int nz = g.nz;
+    const int nz = g.nz, KP = nz + 2;
     const int NQ = (int)g.NQ;
     const int plane = nz * NQ;
     const int NS = (kTX + 2) * (TY + 2);
@@ -908,19 +901,18 @@ __device__ __noinline__ void lines_step(const MDesc &D, int tile) {
 
 // One tile of one solve for the solve's current step; publishes the tile's record.
 template <int NC, int NZM>
-__device__ void tile_step(const MState &S, int tile, bool resident, int TYmax, MHead &hd, unsigned char *smem) {
-    using LY = MLayout<NC, NZM>;
-    constexpr int KP = LY::KP;
+__device__ void tile_step(const MState &S, int tile, bool resident, int TYmax, int nzl, MHead &hd, unsigned char *smem) {
     constexpr int OFF = (NC == 27) ? 1 : 0;  // z row of level 0
-    const LY ly(TYmax, resident);
+    const MLayout<NC, NZM> ly(TYmax, resident, nzl);
     const MDesc &D = hd.D;
     const int TY = D.TY;
     const int NS = (kTX + 2) * (TY + 2), NT = kTX * TY;
     int *smap = reinterpret_cast<int *>(smem + ly.off_map());
     float *sz = reinterpret_cast<float *>(smem + ly.off_z());   // [2][KP][NS]
-    float *srt = reinterpret_cast<float *>(smem + ly.off_rt()); // [2][NZM][NT]
+    float *srt = reinterpret_cast<float *>(smem + ly.off_rt()); // [2][nz][NT]
     const Geom &g = D.g;
     const int nz = (NC == 27) ? g.nz : 1;
+    const int KP = (NC == 27) ? nz + 2 : 1;
     const int NQ = (int)g.NQ;
     const int plane = nz * NQ;
     const int tx = tile % D.tiles_x, ty = tile / D.tiles_x;
@@ -936,7 +928,6 @@ __device__ void tile_step(const MState &S, int tile, bool resident, int TYmax, M
         for (int sl = t; sl < NS; sl += kBlock) smap[sl] = tmap[sl];
         __syncthreads();
     }
-
     if (NC == 27 && NZM <= 16 && D.A64i && (step == MS_INIT || step == MS_BC)) {
         // 3D: x of the tile and halo (updated by this step's d in MS_BC) into shared memory, then
         // the FP64 residual with branch-free couplings
@@ -1085,7 +1076,7 @@ __device__ void tile_step(const MState &S, int tile, bool resident, int TYmax, M
                     ss[u] = (c * KP + k + OFF) * NS + sl;  // the item's z slot in smem
                     const int li = sl % (kTX + 2), lj = sl / (kTX + 2);
                     if (li >= 1 && li <= kTX && lj >= 1 && lj <= TY)  // tile column: keep r for the dots
-                        sr[u] = (c * NZM + k) * NT + (li - 1) + kTX * (lj - 1);
+                        sr[u] = (c * nz + k) * NT + (li - 1) + kTX * (lj - 1);
                     const int v = smap[sl];
                     vv[u] = v;
                     // an update alone (MS_B, MS_UPD) writes only the tile's own columns
@@ -1160,15 +1151,14 @@ __device__ void tile_step(const MState &S, int tile, bool resident, int TYmax, M
                 }
             }
             __syncthreads();
-            if (NC == 27 && (D.precond == 2 || tri)) {  // column tridiagonal solves on tile + halo
-                // one (column, component) per thread while they fit the block: the two
-                // components' recurrences then run side by side instead of one after the other
-                const bool split = 2 * NS <= kBlock;
-                const int nit = split ? 2 * NS : NS;
-                for (int it = t; it < nit; it += kBlock) {
-                    const int c = split ? it / NS : 0, sl = split ? it - c * NS : it;
+            if (NC == 27 && (D.precond == 2 || tri)) {
+                // column tridiagonal solves on tile + halo, one (column, component) at a time, so that
+                // a component's recurrence does not wait for the other's
+                for (int it = t; it < 2 * NS; it += kBlock) {
+                    const int c = it >= NS ? 1 : 0, sl = it - c * NS;
                     const int v = smap[sl];
-                    if (map_live(v)) sia_col<NZM>(D, sz, NS, sl, map_src(v), c, split ? c : 1);
+                    if (map_live(v))
+                        sia_col<NZM>(nz, sz + (c * KP + OFF) * NS + sl, NS, D.pre + c * 3 * plane + map_src(v), plane, NQ);
                 }
                 __syncthreads();
             }
@@ -1287,7 +1277,7 @@ __device__ void tile_step(const MState &S, int tile, bool resident, int TYmax, M
                     Azv[e] = yv[u];
                     zu_out[e] = zu[u];
                     zv_out[e] = zv[u];
-                    const double ru = srt[cc[u]], rv = srt[NZM * NT + cc[u]];
+                    const double ru = srt[cc[u]], rv = srt[nz * NT + cc[u]];
                     p0 += ru * (double)zu[u] + rv * (double)zv[u];
                     p1 += (double)yu[u] * zu[u] + (double)yv[u] * zv[u];
                 }
@@ -1430,10 +1420,10 @@ __device__ bool reduce_wait(MHead &hd, const MDesc *__restrict__ descs, MState *
 template <int NC, int NZM>
 __global__ void __launch_bounds__(kBlock, 2) k_mixed(const MDesc *__restrict__ descs, MState *states,
                                                      const MTile *__restrict__ tiles, int ntiles, int TYmax,
-                                                     int resident, MCtl *ctl, int max_steps) {
+                                                     int resident, int nzl, MCtl *ctl, int max_steps) {
     extern __shared__ __align__(16) unsigned char smem[];
     MHead &hd = *reinterpret_cast<MHead *>(smem);
-    const MLayout<NC, NZM> ly(TYmax, resident != 0);
+    const MLayout<NC, NZM> ly(TYmax, resident != 0, nzl);
     // cache the states of the solves this CTA holds (round robin over the tile list)
     if (threadIdx.x == 0) {
         int n = 0;
@@ -1542,7 +1532,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_mixed(const MDesc *__restrict__ d
                 }
                 __syncthreads();
             }
-            tile_step<NC, NZM>(hd.st[cs], T.tile, resident != 0, TYmax, hd, smem);
+            tile_step<NC, NZM>(hd.st[cs], T.tile, resident != 0, TYmax, nzl, hd, smem);
         }
     }
     // out of steps: fold in the last step's sums so that the next launch resumes exactly
@@ -1610,7 +1600,7 @@ template <int NC, int NZM, bool MULTI = false>
 __global__ void __launch_bounds__(kBlock, 2) k_mixed_dyn(const MDesc *__restrict__ descs, MState *const *states,
                                                          const unsigned *__restrict__ ltick0, int nsolve,
                                                          const MTile *__restrict__ tiles, int ntiles, int TYmax,
-                                                         int TY2max, MCtl *ctl, int max_steps) {
+                                                         int TY2max, int nzl, MCtl *ctl, int max_steps) {
     extern __shared__ __align__(16) unsigned char smem[];
     MHead &hd = *reinterpret_cast<MHead *>(smem);
     __shared__ unsigned long long s_item;
@@ -1698,10 +1688,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_mixed_dyn(const MDesc *__restrict
         if (s_flag == 2) return;
         if (s_flag == 1) continue;
         if (MULTI) {
-            if (hd.D.NC == 27) tile_step<27, NZM>(s_view, T.tile, false, TYmax, hd, smem);
-            else tile_step<9, 1>(s_view, T.tile, false, TY2max, hd, smem);
+            if (hd.D.NC == 27) tile_step<27, NZM>(s_view, T.tile, false, TYmax, nzl, hd, smem);
+            else tile_step<9, 1>(s_view, T.tile, false, TY2max, 1, hd, smem);
         } else {
-            tile_step<NC, NZM>(s_view, T.tile, false, TYmax, hd, smem);
+            tile_step<NC, NZM>(s_view, T.tile, false, TYmax, nzl, hd, smem);
         }
     }
     if (threadIdx.x == 0) s_flag = *(volatile int *)&ctl->abort;

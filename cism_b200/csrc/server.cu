@@ -165,10 +165,10 @@ static int srv_launch_resident(cismgpu_server *S, SrvReq &r) {
     MixedBufs &m = sv.mixed;
     cudaStream_t s = S->es;
     const bool res = mixed_resident(false, 1, r.TY, m.ntiles);
-    const int grid = mixed_launch_grid(false, 1, r.TY, res, m.ntiles);
-    if (grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
+    const MPlan P = mixed_launch_plan(sv, 1, r.TY, res, m.ntiles);
+    if (P.grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
     CU(cudaMemsetAsync(m.ctl, 0, sizeof(MCtl), s));
-    TRY(mixed_dispatch(false, 1, m.desc, m.state, m.tiles, m.ntiles, r.TY, res, m.ctl, S->epoch_steps, grid, s));
+    TRY(mixed_dispatch(false, 1, m.desc, m.state, m.tiles, m.ntiles, r.TY, res, m.ctl, S->epoch_steps, P, s));
     CU(cudaMemcpyAsync(r.h_st, m.state, sizeof(MState), cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(r.h_ctl, m.ctl, sizeof(MCtl), cudaMemcpyDeviceToHost, s));
     return CISMGPU_OK;
@@ -180,7 +180,7 @@ static int srv_launch(cismgpu_server *S, SrvLaunch &L, int cls, bool *multi) {
     const int n = (int)L.members.size();
     *multi = false;
     if (n == 0) return CISMGPU_OK;
-    int TY2 = 1, TY3 = 1, n3 = 0;
+    int TY2 = 1, TY3 = 1, n3 = 0, nzl = 1;
     std::vector<MDesc> descs(n);
     std::vector<MState *> sptr(n);
     std::vector<unsigned> tick(n);
@@ -193,6 +193,7 @@ static int srv_launch(cismgpu_server *S, SrvLaunch &L, int cls, bool *multi) {
         tick[t] = r.tick;
         if (sv.is3d) {
             TY3 = std::max(TY3, r.TY);
+            nzl = std::max(nzl, sv.g.nz);
             ++n3;
         } else {
             TY2 = std::max(TY2, r.TY);
@@ -203,9 +204,9 @@ static int srv_launch(cismgpu_server *S, SrvLaunch &L, int cls, bool *multi) {
     *multi = n3 > 0 && n3 < n;  // class 0 with both kinds: one multi-class launch
     const int nzm = cls == 1 ? 32 : 16;
     const int TYmax = is3d ? TY3 : TY2;
-    const int grid = *multi ? mixed_multi_grid(TY3, TY2) : mixed_dyn_grid(is3d, is3d ? nzm : 1, TYmax);
-    if (grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
-    if ((long long)n > (long long)grid * kMaxCtaSolves) return fail(CISMGPU_EUNSUPPORTED, "too many requests");
+    const MPlan P = mixed_dyn_plan(is3d, is3d ? nzm : 1, TYmax, *multi ? TY2 : 0, nzl);
+    if (P.grid < 1) return fail(CISMGPU_EUNSUPPORTED, "mixed kernel does not fit on an SM at this tile height");
+    if ((long long)n > (long long)P.grid * kMaxCtaSolves) return fail(CISMGPU_EUNSUPPORTED, "too many requests");
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
     const size_t o_d = 0, o_p = al(n * sizeof(MDesc)), o_t = o_p + al(n * sizeof(MState *)),
                  o_l = o_t + al(n * sizeof(unsigned)), o_c = o_l + al(tl.size() * sizeof(MTile)),
@@ -236,16 +237,10 @@ static int srv_launch(cismgpu_server *S, SrvLaunch &L, int cls, bool *multi) {
     std::memcpy(L.h_blk + o_l, tl.data(), tl.size() * sizeof(MTile));
     std::memcpy(L.h_blk + o_c, &c0, sizeof(MCtl));
     CU(cudaMemcpyAsync(base, L.h_blk, o_g, cudaMemcpyHostToDevice, s));
-    if (*multi)
-        TRY(mixed_multi_launch(reinterpret_cast<MDesc *>(base + o_d), reinterpret_cast<MState **>(base + o_p),
-                               reinterpret_cast<unsigned *>(base + o_t), n, reinterpret_cast<MTile *>(base + o_l),
-                               (int)tl.size(), TY3, TY2, reinterpret_cast<MCtl *>(base + o_c), S->epoch_steps, grid,
-                               s));
-    else
-        TRY(mixed_dyn_dispatch(is3d, is3d ? nzm : 1, reinterpret_cast<MDesc *>(base + o_d),
-                               reinterpret_cast<MState **>(base + o_p), reinterpret_cast<unsigned *>(base + o_t), n,
-                               reinterpret_cast<MTile *>(base + o_l), (int)tl.size(), TYmax,
-                               reinterpret_cast<MCtl *>(base + o_c), S->epoch_steps, grid, s));
+    TRY(mixed_dyn_launch(is3d, is3d ? nzm : 1, reinterpret_cast<MDesc *>(base + o_d),
+                         reinterpret_cast<MState **>(base + o_p), reinterpret_cast<unsigned *>(base + o_t), n,
+                         reinterpret_cast<MTile *>(base + o_l), (int)tl.size(), TYmax, *multi ? TY2 : 0,
+                         reinterpret_cast<MCtl *>(base + o_c), S->epoch_steps, P, s));
     k_gather_states<<<(n + 127) / 128, 128, 0, s>>>(reinterpret_cast<MState **>(base + o_p),
                                                    reinterpret_cast<MState *>(base + o_g), n);
     CU(cudaGetLastError());
