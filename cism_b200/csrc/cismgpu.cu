@@ -1246,13 +1246,14 @@ struct Solver {
     // A pointwise statement group (Upd, and a pointwise preconditioner PRE) over every node.
     template <int UPD, int PRE = P_KEEP>
     void node(const double *dgu = nullptr, const double *dgv = nullptr) {
-        k_node<UPD, PRE><<<dim3(nblocks(g.NQ), (unsigned)g.nz), kBlock, 0, stream>>>(g, vargs(), state.as<SolveState>(),
-                                                                                    dgu, dgv);
+        launch_dep(k_node<UPD, PRE>, dim3(nblocks(g.NQ), (unsigned)g.nz), kBlock, 0, stream, g, vargs(),
+                   state.as<SolveState>(), dgu, dgv);
     }
 
     template <int PRE, bool DOT, int NZM>
     void col(const ColArgs &c, RedCtx rc) {
-        k_col<PRE, DOT, NZM><<<nblocks(g.NQ, DOT ? kBlock : 64), DOT ? 2 * kBlock : 128, 0, stream>>>(g, vargs(), c, rc);
+        launch_dep(k_col<PRE, DOT, NZM>, dim3(nblocks(g.NQ, DOT ? kBlock : 64)), DOT ? 2 * kBlock : 128, 0, stream, g,
+                   vargs(), c, rc);
     }
 
     // The staggered halo of one pair of planes.
@@ -1304,14 +1305,14 @@ struct Solver {
             double *T = tri.as<double>();
             const long long NQ = g.NQ;
             if (NCC == 27) {
-                k_tri_lines<true><<<tri_blocks(g), kTriThreads, tri_smem(g), stream>>>(
-                    g, global, p.ru, p.rv, T + TZS_U * NQ, T + TZS_V * NQ, T, st);
+                launch_dep(k_tri_lines<true>, dim3(tri_blocks(g)), kTriThreads, tri_smem(g), stream, g, global, p.ru,
+                           p.rv, T + TZS_U * NQ, T + TZS_V * NQ, T, st);
                 c.zs = T + TZS_U * NQ;
             } else {
                 CU(cudaMemsetAsync(p.zu, 0, NQ * sizeof(double), stream));
                 CU(cudaMemsetAsync(p.zv, 0, NQ * sizeof(double), stream));
-                k_tri_lines<false><<<tri_blocks(g), kTriThreads, tri_smem(g), stream>>>(g, global, p.ru, p.rv, p.zu,
-                                                                                        p.zv, T, st);
+                launch_dep(k_tri_lines<false>, dim3(tri_blocks(g)), kTriThreads, tri_smem(g), stream, g, global, p.ru,
+                           p.rv, p.zu, p.zv, T, st);
                 halo(p.zu, p.zv);
             }
         }

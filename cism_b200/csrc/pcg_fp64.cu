@@ -12,6 +12,34 @@
 namespace cismgpu {
 
 // ---------------------------------------------------------------------------
+// launches of an iteration
+// ---------------------------------------------------------------------------
+// The kernels of an FP64 iteration depend on each other and many last a few microseconds, so the
+// gap between them counts.  They are launched with programmatic dependence: a kernel's blocks are
+// set up while the one before still runs, and wait here for its end (and so for everything before
+// it) before they read anything.  Every kernel launched by launch_dep starts with after_previous.
+// A product of the 31x31x11 dome behind another one: 6.2 -> 4.8 us, SSA 401x401 8.2 -> 6.2.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline void launch_dep(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, A... a) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(a)...);
+}
+
+// ---------------------------------------------------------------------------
 // reduction: per-CTA dd partials -> last CTA finishes with the fixed tree and
 // runs the scalar epilogue
 // ---------------------------------------------------------------------------
@@ -279,6 +307,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_mv_nodes(Geom g, MvMatrix M, cons
                                                         double *__restrict__ ru, double *__restrict__ rv,
                                                         double *__restrict__ T, RedCtx rc) {
     constexpr int NF = (MODE == MV_CG_AZ) ? 2 : 1;
+    after_previous();
     if (rc.st && rc.st->done) return;
     const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
     const int k = blockIdx.y;
@@ -358,11 +387,11 @@ inline void launch_mv(cudaStream_t s, const Geom &g, const MvMatrix &M, const in
                       double *rv, double *T, const RedCtx &rc) {
     const dim3 grid((unsigned)((g.NQ + kBlock - 1) / kBlock), (unsigned)g.nz);
     if (NC == 27 && M.layout == MV_HALF)
-        k_mv_nodes<27, MODE, MV_HALF><<<grid, kBlock, 0, s>>>(g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
+        launch_dep(k_mv_nodes<27, MODE, MV_HALF>, grid, kBlock, 0, s, g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
     else if (M.layout == MV_INNER)
-        k_mv_nodes<NC, MODE, MV_INNER><<<grid, kBlock, 0, s>>>(g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
+        launch_dep(k_mv_nodes<NC, MODE, MV_INNER>, grid, kBlock, 0, s, g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
     else
-        k_mv_nodes<NC, MODE, MV_BOUNDS><<<grid, kBlock, 0, s>>>(g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
+        launch_dep(k_mv_nodes<NC, MODE, MV_BOUNDS>, grid, kBlock, 0, s, g, M, act, xu, xv, yu, yv, bu, bv, ru, rv, T, rc);
 }
 
 // ---------------------------------------------------------------------------
@@ -459,6 +488,7 @@ struct VecArgs {
 template <int UPD, int PRE>
 __global__ void __launch_bounds__(kBlock) k_node(Geom g, VecArgs v, const SolveState *st,
                                                  const double *__restrict__ dgu, const double *__restrict__ dgv) {
+    after_previous();
     if (st->done) return;
     const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
     if (q >= g.NQ) return;
@@ -593,6 +623,7 @@ struct ColArgs {
 // 84k threads of a 201x201 grid spread over all SMs (256 are the reduction's chunk with DOT).
 template <int PRE, bool DOT, int NZM>
 __global__ void __launch_bounds__(DOT ? 2 * kBlock : 128) k_col(Geom g, VecArgs v, ColArgs c, RedCtx rc) {
+    after_previous();
     if (rc.st->done) return;
     constexpr int CW = DOT ? kBlock : 64;
     constexpr int C = kColChunk;
@@ -1134,6 +1165,7 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, c
                                                            const double *__restrict__ bv, double *__restrict__ xu,
                                                            double *__restrict__ xv, const double *__restrict__ T,
                                                            const SolveState *st) {
+    after_previous();
     if (st->done) return;
     extern __shared__ double stri[];  // [b / gamma, sub, 1/denom, omega][line][pitch]
     const int nu = g.jhi - g.jlo + 1, nug = (nu + kTriLines - 1) / kTriLines;
