@@ -307,8 +307,9 @@ static inline unsigned nblocks(long long n, int b = kBlock) { return (unsigned)(
 // 37.0), and the copy costs what three products save.
 constexpr size_t kHalfMinBytes = 64u << 20;
 constexpr int kHalfMinIters = 8;
-// rows of blocks (levels in parallel) for the halo of a matrix's 27 nz coefficient planes
-constexpr unsigned kHaloPlaneRows = 64;
+// rows of blocks (planes in parallel) for the halo of a matrix's 27 nz coefficient planes: with 64 rows each
+// went through 5 planes of an 11-level matrix one after the other, 12.4 us a pair of blocks; now 7.6.
+constexpr unsigned kHaloPlaneRows = 512;
 static inline bool is_check(int iter, int ncheck) { return (iter % ncheck == 0) || iter == 5; }
 
 struct Ptrs {
@@ -590,8 +591,7 @@ struct Solver {
         unsigned long long *out = rsum.as<unsigned long long>();
         cudaStream_t s = stream;
         CU(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s));
-        const long long n = (long long)NC * nvec;
-        const dim3 grid((unsigned)((n + kBlock - 1) / kBlock), 3);
+        const dim3 grid(nblocks(g.NQ), (unsigned)g.nz, is3d ? sym_pairs<27>() : sym_pairs<9>());
         if (is3d)
             k_sym_check<27, true><<<grid, kBlock, 0, s>>>(g, L, act.as<int32_t>(), Auu, Auv, Avu, Avv, out);
         else
@@ -2059,7 +2059,8 @@ static int mixed_reset(Solver &sv, cudaStream_t s) {
     const Ptrs p = sv.ptrs();
     sv.x_current = true;
     CU(cudaMemcpyAsync(p.xu, p.x0u, 2 * sv.nvec * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    k_halo<<<nblocks(4LL * sv.g.NX + 4LL * (sv.g.NY - 4)), kBlock, 0, s>>>(sv.g, p.xu, p.xv, nullptr);
+    k_halo<<<dim3(nblocks(4LL * sv.g.NX + 4LL * (sv.g.NY - 4)), (unsigned)sv.g.nz), kBlock, 0, s>>>(sv.g, p.xu, p.xv,
+                                                                                              nullptr);
     CU(cudaGetLastError());
     CU(cudaMemsetAsync(sv.mixed.vec, 0, (size_t)16 * sv.nvec * sizeof(float), s));
     CU(cudaMemsetAsync(sv.mixed.recs, 0, (size_t)kRecCopies * sv.mixed.ntiles * 2 * sizeof(TileRec), s));  // tags restart at 1
@@ -3576,7 +3577,7 @@ int cismgpu_solver_assemble_system_3d(cismgpu_solver_t *h, int nhalo, double dx,
     cudaStream_t s = sv.stream;
     k_halo<<<dim3(hb, kHaloPlaneRows), kBlock, 0, s>>>(gA, A0, A0 + bs, nullptr);
     k_halo<<<dim3(hb, kHaloPlaneRows), kBlock, 0, s>>>(gA, A0 + 2 * bs, A0 + 3 * bs, nullptr);
-    k_halo<<<hb, kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
+    k_halo<<<dim3(hb, (unsigned)sv.g.nz), kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));
     sv.matrix_changed();
@@ -3656,7 +3657,7 @@ int cismgpu_solver_assemble_system_2d(cismgpu_solver_t *h, int nz, int nhalo, do
     cudaStream_t s = sv.stream;
     k_halo<<<dim3(hb, kHaloPlaneRows), kBlock, 0, s>>>(gA, A0, A0 + bs, nullptr);
     k_halo<<<dim3(hb, kHaloPlaneRows), kBlock, 0, s>>>(gA, A0 + 2 * bs, A0 + 3 * bs, nullptr);
-    k_halo<<<hb, kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
+    k_halo<<<dim3(hb, (unsigned)sv.g.nz), kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));
     sv.matrix_changed();
@@ -3770,7 +3771,7 @@ int cismgpu_solver_assemble_system_2d_diva(
     cudaStream_t s = sv.stream;
     k_halo<<<dim3(hb, kHaloPlaneRows), kBlock, 0, s>>>(gA, A0, A0 + bs, nullptr);
     k_halo<<<dim3(hb, kHaloPlaneRows), kBlock, 0, s>>>(gA, A0 + 2 * bs, A0 + 3 * bs, nullptr);
-    k_halo<<<hb, kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
+    k_halo<<<dim3(hb, (unsigned)sv.g.nz), kBlock, 0, s>>>(sv.g, p.bu, p.bv, nullptr);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));
     sv.matrix_changed();

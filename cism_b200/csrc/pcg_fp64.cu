@@ -859,17 +859,28 @@ __global__ void __launch_bounds__(kBlock) k_resid_vec(Geom g, const int32_t *__r
         int i, j;
         col_of(g, q, i, j);
         const bool on = owned(g, i, j) && act[q] != 0;
-        for (int k = 0; k < g.nz; ++k) {
-            const long long e = (long long)k * g.NQ + q;
-            if (on) {
-                const double r1 = __dsub_rn(yu[e], bu[e]), r2 = __dsub_rn(yv[e], bv[e]);
+        for (int k0 = 0; k0 < g.nz; k0 += kDotChunk) {  // a chunk's loads together, then its terms in order
+            double y1[kDotChunk], y2[kDotChunk], b1[kDotChunk], b2[kDotChunk];
+#pragma unroll
+            for (int u = 0; u < kDotChunk; ++u) {
+                const long long e = (long long)(k0 + u) * g.NQ + q;
+                const bool in = on && k0 + u < g.nz;
+                y1[u] = in ? yu[e] : 0.0;
+                y2[u] = in ? yv[e] : 0.0;
+                b1[u] = in ? bu[e] : 0.0;
+                b2[u] = in ? bv[e] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kDotChunk; ++u) {
+                if (k0 + u >= g.nz) continue;
+                const long long e = (long long)(k0 + u) * g.NQ + q;
+                const double r1 = on ? __dsub_rn(y1[u], b1[u]) : 0.0, r2 = on ? __dsub_rn(y2[u], b2[u]) : 0.0;
                 ru[e] = r1;
                 rv[e] = r2;
-                s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(r1, r1), __dmul_rn(r2, r2)));
-                s1 = dd_add_d(s1, __dadd_rn(__dmul_rn(bu[e], bu[e]), __dmul_rn(bv[e], bv[e])));
-            } else {
-                ru[e] = 0.0;
-                rv[e] = 0.0;
+                if (on) {
+                    s0 = dd_add_d(s0, __dadd_rn(__dmul_rn(r1, r1), __dmul_rn(r2, r2)));
+                    s1 = dd_add_d(s1, __dadd_rn(__dmul_rn(b1[u], b1[u]), __dmul_rn(b2[u], b2[u])));
+                }
             }
         }
     }
@@ -947,30 +958,32 @@ struct SymIdx {
     }
 };
 
-// blockIdx.y: 0 Auu-Auu pairs, 1 Auv-Avu pairs, 2 Avv-Avv pairs; x: coefficient c, level k,
-// column q of the pair's first member.  out[0]: maxdiff as the bits of a non-negative double
+// blockIdx.z: the pairs' kind and the coefficient c of their first member (Auu-Auu and Avv-Avv: c <=
+// NC/2, Auv-Avu: all), blockIdx.y its level, x its column, so that a block reads two runs of
+// columns.  (One flat index over all coefficients, divided by 64-bit sizes per thread and half its
+// threads without a pair, took 276 us on 201x161x11; now 170.)
+// out[0]: maxdiff as the bits of a non-negative double
 // (a NaN difference never wins: "abs(val2 - val1) > maxdiff" is false for it), out[1]: warnings.
+template <int NC>
+__host__ __device__ constexpr int sym_pairs() { return 2 * (NC / 2 + 1) + NC; }
+
 template <int NC, bool FIX>
 __global__ void __launch_bounds__(kBlock) k_sym_check(Geom g, SymIdx L, const int32_t *__restrict__ act,
                                                       double *Auu, double *Auv, double *Avu, double *Avv,
                                                       unsigned long long *out) {
-    const long long n = (long long)g.nz * g.NQ;
-    const long long t = (long long)blockIdx.x * kBlock + threadIdx.x;
-    const int kind = blockIdx.y;
+    constexpr int NH = NC / 2 + 1;
+    const int w = blockIdx.z, k = blockIdx.y;
+    const int kind = w < NH ? 0 : (w < NH + NC ? 1 : 2), c = w - (kind == 0 ? 0 : (kind == 1 ? NH : NH + NC));
+    const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
     unsigned long long dbits = 0ull, nw = 0ull;
-    if (t < NC * n) {
-        const int c = (int)(t / n);
-        const long long r = t - (long long)c * n;
-        const int k = (int)(r / g.NQ);
-        const long long q = r - (long long)k * g.NQ;
-        int i, j;
-        col_of(g, q, i, j);
+    if (q < g.NQ) {
+        const int j = (int)q / g.NX, i = (int)q - j * g.NX;
         const int iA = c % 3 - 1, jA = (c / 3) % 3 - 1, kA = (NC == 27) ? c / 9 - 1 : 0;
         const int cc = NC - 1 - c, cd = NC / 2;
         const int kp = k + kA, ip = i + iA, jp = j + jA;
         // a partner outside the arrays (owned rows at the array edge) is not compared
         const bool inside = kp >= 0 && kp < g.nz && ip >= 0 && ip < g.NX && jp >= 0 && jp < g.NY;
-        if (inside && (kind == 1 || c <= cc)) {
+        if (inside) {
             const long long qp = (long long)jp * g.NX + ip;
             const bool self = kind != 1 && c == cc;  // a diagonal is its own partner
             const bool visA = owned(g, i, j) && act[q] != 0;
