@@ -299,8 +299,10 @@ constexpr int kDotChunk = 8;  // levels whose loads a column's dot terms issue t
 // sums of the early column blocks overlapping the rest of the matvec.  The per-column-block
 // counters sit after the partials and return to zero here.  In 2D a column has one level, so
 // every block reduces its own terms.
+// 2D: five blocks an SM, so that the 638 blocks of a 401x401 grid run at once (three: 99 ms a solve
+// against 87).
 template <int NC, int MODE, int LAY>
-__global__ void __launch_bounds__(kBlock, 3) k_mv_nodes(Geom g, MvMatrix M, const int32_t *__restrict__ act,
+__global__ void __launch_bounds__(kBlock, NC == 9 ? 5 : 3) k_mv_nodes(Geom g, MvMatrix M, const int32_t *__restrict__ act,
                                                         const double *__restrict__ xu, const double *__restrict__ xv,
                                                         double *__restrict__ yu, double *__restrict__ yv,
                                                         const double *__restrict__ bu, const double *__restrict__ bv,
