@@ -1994,7 +1994,7 @@ static int mixed_prepare(Solver &sv, int precond, int TY) {
         const MDesc D = mixed_desc(sv, precond, TY);
         k_slot_maps<<<nblocks((long long)ntiles * NS), kBlock, 0, sv.stream>>>(D, m.maps);
         CU(cudaGetLastError());
-        k_tile_nbrs<<<nblocks(ntiles), kBlock, 0, sv.stream>>>(D, m.maps, m.nbrs);
+        k_tile_nbrs<<<nblocks(32LL * ntiles), kBlock, 0, sv.stream>>>(D, m.maps, m.nbrs);
         CU(cudaGetLastError());
         std::vector<MTile> tl(ntiles);
         for (int t = 0; t < ntiles; ++t) tl[t] = MTile{0, t};
