@@ -7,8 +7,8 @@
 //   blk in {uu, uv, vu, vv}, c the canonical stencil offset
 //   c = (iA+1) + 3(jA+1) + 9(kA+1)  (NC = 27 in 3D; NC = 9 and kA = 0 in 2D),
 //   which is the order the reference's matvec loops run (kA, jA, iA).
-// One thread owns one column and walks its levels; a CTA of 256 threads owns 256
-// consecutive columns.  All loads of matrix planes and vector planes are coalesced.
+// Consecutive threads take consecutive columns (a node each, or a column and its levels), so all
+// loads of matrix planes and vector planes are coalesced.
 //
 // Every global sum uses one fixed reduction tree, independent of launch shape and
 // of other work on the device: per column a double-double sum over k = 1..nz,
