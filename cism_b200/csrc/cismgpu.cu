@@ -144,8 +144,8 @@ static cudaError_t h2d_copy(void *dst, const void *src, size_t bytes, cudaStream
 // an ensemble), and cudaMalloc and cudaFree of their blocks cost milliseconds per handle; so freed
 // blocks are kept, up to kPoolBytes of device memory and kPoolHost pinned blocks in the process, and
 // given to the next handle that fits them.  All of it goes back to the driver when the last handle is
-// gone, and when the device runs out of memory.  As cudaFree does, dev_free waits for the device
-// first, so that a block is idle whichever stream or thread takes it next.  Create, first mixed
+// gone, and when the device runs out of memory.  Only a block whose owner has waited for its stream
+// (idle) is kept; any other is freed by cudaFree, which waits for the device itself.  Create, first mixed
 // solve and close of a 201x201x11 system beside another one: 32.5 ms before (25.3 + 4.1 + 3.1), 25.5 ms now (23.1 + 2.2 + 0.2).
 constexpr size_t kPoolBytes = 4ull << 30;
 constexpr size_t kPoolHostBlock = 4096, kPoolHost = 64;
@@ -203,22 +203,14 @@ struct MemPool {
         *p = b.p;
         return cudaSuccess;
     }
-    void give(void *p) {
+    void give(void *p, bool idle_block) {
         if (!p) return;
-        Blk b;
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            auto it = live.find(p);
-            if (it == live.end()) return;
-            b = it->second;
-            live.erase(it);
-        }
-        int dev = b.dev;
-        if (cudaGetDevice(&dev) == cudaSuccess && dev != b.dev) cudaSetDevice(b.dev);
-        cudaDeviceSynchronize();  // nothing in flight uses the block any more
-        if (dev != b.dev) cudaSetDevice(dev);
         std::lock_guard<std::mutex> lk(mu);
-        if (b.n > kPoolBytes || users == 0) {
+        auto it = live.find(p);
+        if (it == live.end()) return;
+        const Blk b = it->second;
+        live.erase(it);
+        if (!idle_block || b.n > kPoolBytes || users == 0) {
             cudaFree(b.p);
             return;
         }
@@ -241,11 +233,10 @@ struct MemPool {
         }
         return cudaHostAlloc(p, kPoolHostBlock, cudaHostAllocPortable);
     }
-    void give_host(void *p) {
+    void give_host(void *p, bool idle_block) {
         if (!p) return;
-        cudaDeviceSynchronize();
         std::lock_guard<std::mutex> lk(mu);
-        if (host.size() < kPoolHost && users > 0) host.push_back(p);
+        if (idle_block && host.size() < kPoolHost && users > 0) host.push_back(p);
         else cudaFreeHost(p);
     }
     void join() {
@@ -262,7 +253,7 @@ static MemPool &mem_pool() {
     return *pool;
 }
 cudaError_t dev_alloc(void **p, size_t bytes) { return mem_pool().take(p, bytes); }
-void dev_free(void *p) { mem_pool().give(p); }
+void dev_free(void *p, bool idle) { mem_pool().give(p, idle); }
 
 struct DevBuf {
     void *p = nullptr;
@@ -275,8 +266,8 @@ struct DevBuf {
         else p = nullptr;
         return e;
     }
-    void release() {
-        if (p) dev_free(p);
+    void release(bool idle = false) {  // idle: the caller has waited for the block's last use
+        if (p) dev_free(p, idle);
         p = nullptr;
         n = 0;
     }
@@ -411,26 +402,27 @@ struct Solver {
     Solver &operator=(const Solver &) = delete;
 
     void destroy() {
-        A.release(); raw.release(); vec.release(); act.release(); partials.release(); state.release(); map.release();
-        tri.release();
-        sia.release();
-        half.release();
-        terms.release();
+        const bool idle = !stream || cudaStreamSynchronize(stream) == cudaSuccess;
+        A.release(idle); raw.release(idle); vec.release(idle); act.release(idle); partials.release(idle); state.release(idle); map.release(idle);
+        tri.release(idle);
+        sia.release(idle);
+        half.release(idle);
+        terms.release(idle);
         half_state = -1;
-        A_sav.release();
-        x_sav.release();
-        rsum.release();
-        asm_in.release();
-        asm_k.release();
-        bc_in.release();
-        diva_in.release();
-        diva_eq[0].release();
-        diva_eq[1].release();
+        A_sav.release(idle);
+        x_sav.release(idle);
+        rsum.release(idle);
+        asm_in.release(idle);
+        asm_k.release(idle);
+        bc_in.release(idle);
+        diva_in.release(idle);
+        diva_eq[0].release(idle);
+        diva_eq[1].release(idle);
         diva_valid = false;
         have_sav = false;
-        mixed.release();
-        rprod.release();
-        if (h_done) mem_pool().give_host(h_done);  // h_state with it
+        mixed.release(idle);
+        rprod.release(idle);
+        if (h_done) mem_pool().give_host(h_done, idle);  // h_state with it
         h_done = nullptr;
         h_state = nullptr;
         for (auto &e : ev) if (e) cudaEventDestroy(e), e = nullptr;
@@ -1975,10 +1967,10 @@ static int mixed_prepare(Solver &sv, int precond, int TY) {
         const int ntiles = tiles_for(g, TY);
         const int NS = (kTX + 2) * (TY + 2);
         if (ntiles > m.ntiles_cap || (long long)ntiles * NS > m.maps_cap) {
-            if (m.recs) dev_free(m.recs);
-            if (m.maps) dev_free(m.maps);
-            if (m.nbrs) dev_free(m.nbrs);
-            if (m.tiles) dev_free(m.tiles);
+            if (m.recs) dev_free(m.recs, false);
+            if (m.maps) dev_free(m.maps, false);
+            if (m.nbrs) dev_free(m.nbrs, false);
+            if (m.tiles) dev_free(m.tiles, false);
             m.recs = nullptr;
             m.maps = nullptr;
             m.nbrs = nullptr;
@@ -2702,7 +2694,7 @@ struct MixedBatch {
     MState *h_states = nullptr;  // pinned
     MCtl *h_ctl = nullptr;       // pinned
     void release() {
-        if (dmem) dev_free(dmem);
+        if (dmem) dev_free(dmem, false);
         if (h_states) cudaFreeHost(h_states);
         if (h_ctl) cudaFreeHost(h_ctl);
         dmem = nullptr;

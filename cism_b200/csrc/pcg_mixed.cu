@@ -1796,8 +1796,8 @@ __global__ void k_tri_to_f32(Geom g, const double *__restrict__ T, float *__rest
     }
 }
 
-// The handles' device memory (cismgpu.cu).
-void dev_free(void *p);
+// The handles' device memory (cismgpu.cu); idle: nothing in flight uses the block.
+void dev_free(void *p, bool idle);
 
 // Device buffers of the mixed solver for one system (owned by the host Solver).
 struct MixedBufs {
@@ -1825,10 +1825,10 @@ struct MixedBufs {
     int ntiles = 0;
     int ntiles_cap = 0;
     long long maps_cap = 0;
-    void release() {
+    void release(bool idle = false) {
         for (void *p : {(void *)A32, (void *)A64i, (void *)pre, (void *)vec, (void *)recs, (void *)state, (void *)desc,
                         (void *)tiles, (void *)ctl, (void *)maps, (void *)nbrs, (void *)bc, (void *)tri})
-            if (p) dev_free(p);
+            if (p) dev_free(p, idle);
         tri = nullptr;
         A32 = nullptr;
         A64i = nullptr;

@@ -269,11 +269,12 @@ static void srv_deliver(cismgpu_server *S, SrvReq &r, int status, double err, in
 
 // The handle of a delivered request freed and its bytes returned to the budget.
 static void srv_free(cismgpu_server *S, SrvReq &r) {
+    const bool idle = cudaStreamSynchronize(S->es) == cudaSuccess;  // no epoch uses the request's buffers
     if (r.h) {
         cismgpu_solver_destroy(r.h);
         r.h = nullptr;
     }
-    if (r.h_st) mem_pool().give_host(r.h_st);
+    if (r.h_st) mem_pool().give_host(r.h_st, idle);
     r.h_st = nullptr;
     r.h_ctl = nullptr;
     std::lock_guard<std::mutex> lk(S->mu);
