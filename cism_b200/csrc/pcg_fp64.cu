@@ -1165,6 +1165,8 @@ __global__ void k_tri_factor(Geom g, int global, double *__restrict__ T, SolveSt
 // Line solves of tridiag_solver_local_2d (:4985-5013 u, :5041-5069 v) from planes bu, bv into
 // xu, xv, which hold zeros outside the lines: gamma forward, then back substitution.  SUM (3D): the
 // right-hand side is the sum of r over the levels, in level order (tridiag_solver_local_3d :4585-4590).
+// pending: the halo update of b is still to come (U_RHALO, by the kernel that follows); it may reach
+// owned positions (no_ice zeroes the last owned row and column), so the lines read what it will leave.
 // A line is a chain of dependent FP64 operations (three a position forward, two backward), which
 // bounds the launch; so everything else is taken off the chain: a block stages kTriLines lines,
 // kTriChunk positions at a time, in shared memory with all its threads (coalesced for the u lines,
@@ -1176,7 +1178,7 @@ constexpr int kTriLines = 4, kTriChunk = 376, kTriThreads = 128;
 static_assert(4 * kTriLines * (kTriChunk + 1) * sizeof(double) <= 48 * 1024, "no opt-in shared memory");
 
 template <bool SUM>
-__global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, const double *__restrict__ bu,
+__global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, int pending, const double *__restrict__ bu,
                                                            const double *__restrict__ bv, double *__restrict__ xu,
                                                            double *__restrict__ xv, const double *__restrict__ T,
                                                            const SolveState *st) {
@@ -1206,18 +1208,23 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, c
     for (int c = 0; c < nch; ++c) {
         const int c0 = c * kTriChunk, n = min(kTriChunk, len - c0);
         each(c0, n, [&](int w, long long e) {
+            long long f = e;
+            if (pending) {
+                const int j = (int)e / g.NX, i = (int)e - j * g.NX;
+                f = halo_src(g, i, j, e);
+            }
             double v = 0.0;
-            if (SUM) {
+            if (SUM && f >= 0) {
                 for (int k0 = 0; k0 < g.nz; k0 += 8) {
                     double r[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) r[u] = (k0 + u < g.nz) ? b[(long long)(k0 + u) * g.NQ + e] : 0.0;
+                    for (int u = 0; u < 8; ++u) r[u] = (k0 + u < g.nz) ? b[(long long)(k0 + u) * g.NQ + f] : 0.0;
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
                         if (k0 + u < g.nz) v = __dadd_rn(v, r[u]);
                 }
-            } else {
-                v = b[e];
+            } else if (f >= 0) {
+                v = b[f];
             }
             sb[w] = v;
             ss[w] = sub[e];
