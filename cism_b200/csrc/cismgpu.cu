@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "mempool.h"
 #include "pcg_fp64.cu"
 #include "pcg_mixed.cu"
 #include "assembly.cu"
@@ -140,119 +141,24 @@ static cudaError_t h2d_copy(void *dst, const void *src, size_t bytes, cudaStream
     return cudaSuccess;
 }
 
-// Memory of the handles.  Systems come and go with the same sizes (served requests, the members of
-// an ensemble), and cudaMalloc and cudaFree of their blocks cost milliseconds per handle; so freed
-// blocks are kept, up to kPoolBytes of device memory and kPoolHost pinned blocks in the process, and
-// given to the next handle that fits them.  All of it goes back to the driver when the last handle is
-// gone, and when the device runs out of memory.  Only a block whose owner has waited for its stream
-// (idle) is kept; any other is freed by cudaFree, which waits for the device itself.  Create, first mixed
-// solve and close of a 201x201x11 system beside another one: 32.5 ms before (25.3 + 4.1 + 3.1), 25.5 ms now (23.1 + 2.2 + 0.2).
-constexpr size_t kPoolBytes = 4ull << 30;
-constexpr size_t kPoolHostBlock = 4096, kPoolHost = 64;
-
-struct MemPool {
-    struct Blk {
-        void *p;
-        size_t n;
-        int dev;
-    };
-    std::mutex mu;
-    std::vector<Blk> idle;                // freed device blocks, oldest first
-    size_t held = 0;                      // their bytes
-    std::map<void *, Blk> live;           // blocks handed out
-    std::vector<void *> host;             // freed pinned blocks of kPoolHostBlock bytes
-    int users = 0;
-
-    void trim() {  // caller holds mu
-        for (const Blk &b : idle) cudaFree(b.p);
-        for (void *h : host) cudaFreeHost(h);
-        idle.clear();
-        host.clear();
-        held = 0;
-    }
-    cudaError_t take(void **p, size_t bytes) {
-        const size_t unit = bytes >= (1u << 20) ? (1u << 20) : 512;
-        const size_t n = std::max(unit, (bytes + unit - 1) / unit * unit);
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return e;
-        std::lock_guard<std::mutex> lk(mu);
-        size_t best = idle.size();
-        for (size_t k = 0; k < idle.size(); ++k)  // the smallest that fits without wasting a quarter
-            if (idle[k].dev == dev && idle[k].n >= n && idle[k].n - n <= n / 4 &&
-                (best == idle.size() || idle[k].n < idle[best].n))
-                best = k;
-        Blk b{nullptr, n, dev};
-        if (best < idle.size()) {
-            b = idle[best];
-            idle.erase(idle.begin() + best);
-            held -= b.n;
-        } else {
-            e = cudaMalloc(&b.p, n);
-            if (e == cudaErrorMemoryAllocation && !idle.empty()) {
-                (void)cudaGetLastError();
-                trim();
-                e = cudaMalloc(&b.p, n);
-            }
-            if (e != cudaSuccess) {
-                *p = nullptr;
-                return e;
-            }
-        }
-        live[b.p] = b;
-        *p = b.p;
-        return cudaSuccess;
-    }
-    void give(void *p, bool idle_block) {
-        if (!p) return;
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = live.find(p);
-        if (it == live.end()) return;
-        const Blk b = it->second;
-        live.erase(it);
-        if (!idle_block || b.n > kPoolBytes || users == 0) {
-            cudaFree(b.p);
-            return;
-        }
-        while (held + b.n > kPoolBytes) {  // the oldest make room
-            cudaFree(idle.front().p);
-            held -= idle.front().n;
-            idle.erase(idle.begin());
-        }
-        idle.push_back(b);
-        held += b.n;
-    }
-    cudaError_t take_host(void **p) {
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            if (!host.empty()) {
-                *p = host.back();
-                host.pop_back();
-                return cudaSuccess;
-            }
-        }
-        return cudaHostAlloc(p, kPoolHostBlock, cudaHostAllocPortable);
-    }
-    void give_host(void *p, bool idle_block) {
-        if (!p) return;
-        std::lock_guard<std::mutex> lk(mu);
-        if (idle_block && host.size() < kPoolHost && users > 0) host.push_back(p);
-        else cudaFreeHost(p);
-    }
-    void join() {
-        std::lock_guard<std::mutex> lk(mu);
-        ++users;
-    }
-    void leave() {
-        std::lock_guard<std::mutex> lk(mu);
-        if (--users == 0) trim();
+// The handles' memory (mempool.h) on the CUDA runtime.
+struct CudaDriver {
+    static int device(int *dev) { return cudaGetDevice(dev); }
+    static int alloc(void **p, size_t bytes) { return cudaMalloc(p, bytes); }
+    static void release(void *p) { cudaFree(p); }
+    static int alloc_host(void **p, size_t bytes) { return cudaHostAlloc(p, bytes, cudaHostAllocPortable); }
+    static void release_host(void *p) { cudaFreeHost(p); }
+    static bool out_of_memory(int e) {
+        if (e != cudaErrorMemoryAllocation) return false;
+        (void)cudaGetLastError();
+        return true;
     }
 };
-static MemPool &mem_pool() {
-    static MemPool *pool = new MemPool();  // never destroyed: handles may outlive static destructors
+static MemPool<CudaDriver> &mem_pool() {
+    static auto *pool = new MemPool<CudaDriver>();  // never destroyed: handles may outlive static destructors
     return *pool;
 }
-cudaError_t dev_alloc(void **p, size_t bytes) { return mem_pool().take(p, bytes); }
+cudaError_t dev_alloc(void **p, size_t bytes) { return (cudaError_t)mem_pool().take(p, bytes); }
 void dev_free(void *p, bool idle) { mem_pool().give(p, idle); }
 
 struct DevBuf {
@@ -443,7 +349,7 @@ struct Solver {
             CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
             own_stream = true;
         }
-        CU(mem_pool().take_host((void **)&h_done));
+        CU((cudaError_t)mem_pool().take_host((void **)&h_done));
         h_state = reinterpret_cast<SolveState *>(reinterpret_cast<char *>(h_done) + 256);
         static_assert(256 + sizeof(SolveState) <= kPoolHostBlock, "the polling flags and the state share a block");
         CU(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));

@@ -139,7 +139,7 @@ static int srv_admit(SrvReq &r) {
         if (owned >= kSrvResidentMin) {
             r.cls = 2;
             r.TY = ty1;
-            CU(mem_pool().take_host((void **)&r.h_st));  // one pinned block for both
+            CU((cudaError_t)mem_pool().take_host((void **)&r.h_st));  // one pinned block for both
             r.h_ctl = reinterpret_cast<MCtl *>(reinterpret_cast<char *>(r.h_st) + 1024);
             static_assert(sizeof(MState) <= 1024 && 1024 + sizeof(MCtl) <= kPoolHostBlock, "one block");
         }
