@@ -299,10 +299,15 @@ struct Solver {
     double prof_bytes = 0.0;
     int last_ty = 0;  // tile height of the last mixed solve
 
-    Solver() { mem_pool().join(); }
+    // pooled: memory that handles free is kept while this solver lives.  Not for the one-shot calls'
+    // cached solver, which lives as long as the process.
+    const bool pooled;
+    explicit Solver(bool keeps_pool = true) : pooled(keeps_pool) {
+        if (pooled) mem_pool().join();
+    }
     ~Solver() {
         destroy();
-        mem_pool().leave();
+        if (pooled) mem_pool().leave();
     }
     Solver(const Solver &) = delete;
     Solver &operator=(const Solver &) = delete;
@@ -2343,7 +2348,7 @@ static int oneshot_solve(int alg, bool is3d, int nx, int ny, int nz, const cismg
     TRY(validate(nx, ny, is3d ? nz : 1, par, indx, act, Auu, Auv, Avu, Avv, bu, bv));
     TRY(validate_solve_args(precond, ncheck, maxiters));
     TRY(validate_indx(indx, is3d ? 27 : 9));
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     const double *blocks[4] = {Auu, Auv, Avu, Avv};
@@ -2366,7 +2371,7 @@ static int oneshot_matvec(bool is3d, int nx, int ny, int nz, const cismgpu_par_t
     TRY(validate(nx, ny, is3d ? nz : 1, par, indx, act, Auu, Auv, Avu, Avv, xu, xv));
     TRY(validate_indx(indx, is3d ? 27 : 9));
     if (!yu || !yv) return fail(CISMGPU_EINVAL, "null output pointer");
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     const double *blocks[4] = {Auu, Auv, Avu, Avv};
@@ -2395,7 +2400,7 @@ static int oneshot_resid_vec(bool is3d, int nx, int ny, int nz, const cismgpu_pa
     TRY(validate(nx, ny, is3d ? nz : 1, par, indx, act, Auu, Auv, Avu, Avv, bu, bv));
     TRY(validate_indx(indx, is3d ? 27 : 9));
     if (!uvel || !vvel || !resid_u || !resid_v || !L2_norm) return fail(CISMGPU_EINVAL, "null pointer argument");
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     const double *blocks[4] = {Auu, Auv, Avu, Avv};
@@ -2418,7 +2423,7 @@ static int oneshot_symmetry(bool is3d, int nx, int ny, int nz, const cismgpu_par
         return fail(CISMGPU_EINVAL, "null pointer argument");
     TRY(validate_geom(nx, ny, is3d ? nz : 1, par));
     TRY(validate_indx(indx, is3d ? 27 : 9));
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     TRY(sv.set_geom(make_geom(nx, ny, is3d ? nz : 1, par), is3d));
@@ -2482,7 +2487,7 @@ static int oneshot_assemble(bool three_d, int nx, int ny, int nz, int nhalo, con
     cismgpu_par_t par{};
     par.staggered_ilo = 1; par.staggered_ihi = nx - 1; par.staggered_jlo = 1; par.staggered_jhi = ny - 1;
     par.tasks_row = par.tasks_col = 1;
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     TRY(sv.set_geom(make_geom(nx, ny, three_d ? nz : 1, &par), three_d));
@@ -2512,7 +2517,7 @@ static int oneshot_resid_velo(bool is3d, int whichresid, int nx, int ny, int nz,
     g_last_error.clear();
     if (!uvel || !vvel || !usav || !vsav || !resid_velo) return fail(CISMGPU_EINVAL, "null pointer argument");
     TRY(validate_geom(nx, ny, is3d ? nz : 1, par));
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     TRY(sv.set_geom(make_geom(nx, ny, is3d ? nz : 1, par), is3d));
@@ -2538,7 +2543,7 @@ static int oneshot_global_sum(int nx, int ny, int nz, const cismgpu_par_t *par, 
     if (par->staggered_ilo < 1 || par->staggered_ihi > nx - 1 || par->staggered_ilo > par->staggered_ihi ||
         par->staggered_jlo < 1 || par->staggered_jhi > ny - 1 || par->staggered_jlo > par->staggered_jhi)
         return fail(CISMGPU_EINVAL, "owned vertex bounds outside the array");
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     const Geom g = make_geom(nx, ny, nz, par);
@@ -3154,7 +3159,7 @@ static int oneshot_boundary3d(int which, int nx, int ny, int nz, int nhalo, doub
     cismgpu_par_t par{};
     par.staggered_ilo = 1; par.staggered_ihi = nx - 1; par.staggered_jlo = 1; par.staggered_jhi = ny - 1;
     par.tasks_row = par.tasks_col = 1;
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     TRY(sv.set_geom(make_geom(nx, ny, nz, &par), true));
@@ -3221,7 +3226,7 @@ static int oneshot_boundary2d(int which, int nx, int ny, int nhalo, double dx, d
     cismgpu_par_t par{};
     par.staggered_ilo = 1; par.staggered_ihi = nx - 1; par.staggered_jlo = 1; par.staggered_jhi = ny - 1;
     par.tasks_row = par.tasks_col = 1;
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     TRY(sv.set_geom(make_geom(nx, ny, 1, &par), false));
@@ -3280,7 +3285,7 @@ static int oneshot_assemble_diva(int nx, int ny, int nz, int nhalo, const double
     cismgpu_par_t par{};
     par.staggered_ilo = 1; par.staggered_ihi = nx - 1; par.staggered_jlo = 1; par.staggered_jhi = ny - 1;
     par.tasks_row = par.tasks_col = 1;
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     TRY(sv.set_geom(make_geom(nx, ny, 1, &par), false));
@@ -3347,7 +3352,7 @@ int cismgpu_load_vector_gravity(int nx, int ny, int nz, int nhalo, const double 
     cismgpu_par_t par{};
     par.staggered_ilo = 1; par.staggered_ihi = nx - 1; par.staggered_jlo = 1; par.staggered_jhi = ny - 1;
     par.tasks_row = par.tasks_col = 1;
-    if (!g_oneshot) g_oneshot = new Solver();
+    if (!g_oneshot) g_oneshot = new Solver(false);
     Solver &sv = *g_oneshot;
     TRY(sv.init(nullptr));
     TRY(sv.set_geom(make_geom(nx, ny, nz, &par), true));

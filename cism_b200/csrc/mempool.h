@@ -3,8 +3,8 @@
 // Systems come and go with the same sizes (served requests, the members of an ensemble), and cudaMalloc
 // and cudaFree of their blocks cost milliseconds per handle; so freed blocks are kept, up to kPoolBytes
 // of device memory and kPoolHost pinned blocks in the process, and given to the next handle that fits
-// them.  All of it goes back to the driver when the last user is gone, and when an allocation of the
-// library runs out of memory.
+// them.  All of it goes back to the driver when the last handle or server is gone (the one-shot
+// calls' cached solver does not count), and when an allocation of the library runs out of memory.
 // Only a block whose owner has waited for its last use (idle) is kept; any other is freed by cudaFree,
 // which waits for the device itself.
 //
