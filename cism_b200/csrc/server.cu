@@ -296,6 +296,7 @@ static void srv_admit_loop(cismgpu_server *S) {
     cudaSetDevice(S->device);
     for (;;) {
         SrvReq *r = nullptr;
+        size_t room = 0;  // of the budget, beside the admitted requests
         {
             std::unique_lock<std::mutex> lk(S->mu);
             S->cv.wait(lk, [&] {
@@ -312,7 +313,9 @@ static void srv_admit_loop(cismgpu_server *S) {
                 S->used += r->bytes;
             }
             S->uploading += 1;
+            room = S->budget - S->used;
         }
+        mem_pool().shrink(room);  // what finished requests left counts as well
         int rc = r->bytes == 0 ? fail(CISMGPU_ENOMEM, "request larger than the HBM budget") : srv_admit(*r);
         {
             std::lock_guard<std::mutex> lk(S->mu);

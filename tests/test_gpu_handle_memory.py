@@ -65,3 +65,24 @@ assert used() - base > 100 * MB
 s.close()
 assert used() - base < 8 * MB, (used() - base) / MB
 """)
+
+
+def test_server_budget_counts_what_requests_leave(gpu_lib):
+    """Requests of falling sizes, whose blocks do not fit the next one, through a budget that holds the largest."""
+    run("""
+probs = [asm.ice_stream(n, n - 3, 11, seed=n) for n in (96, 84, 73, 64, 55)]
+def nbytes(P):  # an upper bound of the largest request's bytes, as the server counts them
+    return (P.nx - 1) * (P.ny - 1) * P.nz * (4 * 27 * 8 * 2 + 27 * 8 + 27 * 16 + 16 * 8 + 88) + 9 * MB
+budget = nbytes(probs[0])
+base = used()
+srv = cg.Server(hbm_budget_bytes=budget)
+peak = 0
+for P in probs:
+    rid = srv.submit(P, precond=2, ncheck=5, tol=1e-6, maxiters=200)
+    srv.drain()
+    assert srv.poll(rid)["done"]
+    peak = max(peak, used() - base)
+srv.close()
+assert peak < budget + 16 * MB, (peak / MB, budget / MB)
+assert used() - base < 8 * MB
+""")
