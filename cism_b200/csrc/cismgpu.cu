@@ -2971,10 +2971,13 @@ int cismgpu_solver_solve_batch(cismgpu_solver_t **solvers, int n, int algorithm,
         B.svs.push_back(&solvers[t]->sv);
     }
     cudaStream_t s = cuda_stream ? (cudaStream_t)cuda_stream : B.svs[0]->stream;
-    TRY(tune_batch_floor(B.svs, precond, linear_solve_ncheck, s));
-    TRY(batch_prepare(B, precond, linear_solve_ncheck, tolerance, maxiters));
-    TRY(batch_enqueue(B, s));
-    CU(cudaStreamSynchronize(s));
+    int rc = tune_batch_floor(B.svs, precond, linear_solve_ncheck, s);
+    if (!rc) rc = batch_prepare(B, precond, linear_solve_ncheck, tolerance, maxiters);
+    if (!rc) rc = batch_enqueue(B, s);
+    // also after an error: what was queued on s uses the members' buffers, which their own streams do not cover
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (rc) return rc;
+    CU(e);
     return batch_results(B, errs, niters, statuses);
 }
 
