@@ -313,8 +313,7 @@ struct Solver {
     Solver &operator=(const Solver &) = delete;
 
     void destroy() {
-        // a caller's stream may be gone or capturing by now: it is left alone, and cudaFree waits instead
-        const bool idle = !stream || (own_stream && cudaStreamSynchronize(stream) == cudaSuccess);
+        const bool idle = !stream || cudaStreamSynchronize(stream) == cudaSuccess;
         A.release(idle); raw.release(idle); vec.release(idle); act.release(idle); partials.release(idle); state.release(idle); map.release(idle);
         tri.release(idle);
         sia.release(idle);

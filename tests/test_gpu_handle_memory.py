@@ -86,20 +86,3 @@ srv.close()
 assert peak < budget + 16 * MB, (peak / MB, budget / MB)
 assert used() - base < 8 * MB
 """)
-
-
-def test_handle_outlives_its_callers_stream(gpu_lib):
-    """A handle on a caller's stream is closed after the stream was destroyed."""
-    run("""
-import ctypes
-rt = ctypes.CDLL([l.split()[-1] for l in open("/proc/self/maps") if "libcudart" in l][0])
-st = ctypes.c_void_p()
-assert rt.cudaStreamCreateWithFlags(ctypes.byref(st), 1) == 0
-s = cg.DeviceSolver(small, stream=st.value)
-want = s.solve(cg.ALG_CHRONGEAR, 2, 5, 1e-8, 100), s.x()
-assert rt.cudaStreamDestroy(st) == 0
-s.close()
-s = solve(small)
-got = s.solve(cg.ALG_CHRONGEAR, 2, 5, 1e-8, 100), s.x()
-assert got[0] == want[0] and np.array_equal(got[1][0], want[1][0])
-""")
