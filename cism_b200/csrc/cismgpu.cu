@@ -1119,6 +1119,7 @@ struct Solver {
         CU(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
         CU(cudaStreamSynchronize(stream));
         half_state = h == 0 ? 1 : 0;
+        if (half_state == 0) half.release(true);  // unused, and the stream has been waited for: kept for the next matrix
         return CISMGPU_OK;
     }
 
@@ -1859,13 +1860,9 @@ static int mixed_prepare(Solver &sv, int precond, int TY) {
             (void)cudaGetLastError();
             m.sym = rc == CISMGPU_OK && sv.half_state == 1;
         }
-        if (NC == 27 && !m.sym) {
-            sv.half.release();
-            sv.half_state = 0;
-            if (!m.A64i) {
-                CU(dev_alloc((void **)&m.A64i, (size_t)NC * nvec * 2 * sizeof(double2)));
-                m.nbytes += (size_t)NC * nvec * 2 * sizeof(double2);
-            }
+        if (NC == 27 && !m.sym && !m.A64i) {
+            CU(dev_alloc((void **)&m.A64i, (size_t)NC * nvec * 2 * sizeof(double2)));
+            m.nbytes += (size_t)NC * nvec * 2 * sizeof(double2);
         }
         m.il = !m.sym && m.A64i != nullptr;
         if (NC == 27 && !m.sym) k_to_f32<27><<<1184, kBlock, 0, sv.stream>>>(g, sv.A.as<double>(), m.A32, m.A64i);

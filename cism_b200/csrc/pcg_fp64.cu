@@ -254,13 +254,14 @@ __device__ __forceinline__ void mv_row(const Geom &g, const MvMatrix &M, const d
 // Auu, Auv with Avu, Avv with Avv, bit for bit), which check_symmetry_assembled_matrix_3d averages
 // to equality before every 3D solve (glissade_velo_higher.F90:2923-2931).  No owned vertex may lie
 // on the edge of the array (a partner is then always inside).  a32 (may be null): the same half
-// as FP32.  One thread per node and stored coupling; every plane is read once, coalesced: 201x201x11
-// 98 us for the test and the FP64 half, where the mixed solver's test with one thread per column and its
-// copy took 299 + 93 us.
+// as FP32.  One thread per node and stored coupling; every plane is read once, coalesced (201x201x11: 98 us
+// for the test and the FP64 half).  Once a difference is known the copy is of no use, and the blocks
+// that have not started yet end at once; a block may still read an old flag, and then does its part in vain.
 __global__ void __launch_bounds__(kBlock) k_half3d(Geom g, const int32_t *__restrict__ act, const double *__restrict__ A,
                                                    double *__restrict__ H, float4 *__restrict__ a32, int *flag) {
     const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
     const int k = blockIdx.y, h = blockIdx.z, c = 13 + h;
+    if (*flag != 0) return;
     bool bad = false;
     if (q < g.NQ) {
         const int i = (int)(q % g.NX), j = (int)(q / g.NX);
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kBlock) k_half3d(Geom g, const int32_t *__rest
         reinterpret_cast<Dbl4 *>(H)[h * plane + e] = a;
         if (a32) a32[h * plane + e] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
     }
-    if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
+    if (bad) *flag = 1;
 }
 
 enum MvMode { MV_PLAIN = 0, MV_RESID, MV_DQ, MV_CG_AZ };
