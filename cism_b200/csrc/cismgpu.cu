@@ -268,9 +268,7 @@ struct Solver {
     DevBuf A, raw, vec, act, partials, state, map;
     DevBuf tri;       // tridiagonal preconditioner planes (TriPlane), on first use
     DevBuf half;      // symmetric half of a 3D matrix (k_half3d), on first use
-    DevBuf terms;     // dot terms of a 3D matvec ([2][nz][NQ])
     int half_state = -1;  // half holds the current matrix: 1; not exactly symmetric: 0; not tested: -1
-    DevBuf sia;       // column pivots of the FP64 solvers (k_sia_factor), on first use
     DevBuf A_sav, x_sav;      // accelerated Picard's saved matrix and velocity (cismgpu_solver_save)
     DevBuf rsum;              // the reproducible sum's exponent extremes and level sums
     DevBuf rprod;             // reproducible-sum solves: the two product fields and the flag
@@ -316,9 +314,7 @@ struct Solver {
         const bool idle = !stream || cudaStreamSynchronize(stream) == cudaSuccess;
         A.release(idle); raw.release(idle); vec.release(idle); act.release(idle); partials.release(idle); state.release(idle); map.release(idle);
         tri.release(idle);
-        sia.release(idle);
         half.release(idle);
-        terms.release(idle);
         half_state = -1;
         A_sav.release(idle);
         x_sav.release(idle);
@@ -1095,6 +1091,10 @@ struct Solver {
         return CISMGPU_OK;
     }
 
+    static bool tri_precond(int precond) {
+        return precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
+    }
+
     // A, or the array it lives in, has changed: the copies made from it are stale.
     void matrix_changed() {
         mixed.stale = true;
@@ -1123,11 +1123,18 @@ struct Solver {
         return CISMGPU_OK;
     }
 
-    // The matvecs of an FP64 solve read the symmetric half where that pays: a matrix that L2
-    // does not keep (kHalfMinBytes) and enough iterations for its test and copy.  A device without
-    // room for the copy reads the planes.
-    int matrix_setup(int maxiters) {
-        if (is3d) CU(terms.ensure((size_t)2 * nvec * sizeof(double)));
+    // Work arrays of an FP64 3D solve, in the block that stages uploads and downloads (216 bytes a node,
+    // idle meanwhile): the dot terms of a matvec ([2][nz][NQ]), then the column pivots ([4][nz][NQ]).
+    double *dot_terms() const { return is3d ? raw.as<double>() : nullptr; }
+    double *column_pivots() const { return raw.as<double>() + 2 * nvec; }
+
+    // The memory of an FP64 solve and the matrix its matvecs read.  What the solve cannot do without comes
+    // first.  Then the symmetric half, where it pays: a matrix that L2 does not keep (kHalfMinBytes) and
+    // a caller that allows enough iterations (kHalfMinIters); a device without room for it reads the planes.
+    int matrix_setup(int precond, int maxiters) {
+        if (is3d) CU(raw.ensure((size_t)6 * nvec * sizeof(double)));
+        if (tri_precond(precond)) CU(tri.ensure((size_t)NTRI * g.NQ * sizeof(double)));
+        if (repro) CU(rprod.ensure((size_t)2 * nvec * sizeof(double) + 256));
         if (!is3d || half_state >= 0 || !inner_geometry() || maxiters < kHalfMinIters ||
             (size_t)108 * nvec * sizeof(double) < kHalfMinBytes)
             return CISMGPU_OK;
@@ -1166,23 +1173,19 @@ struct Solver {
             g, u, v, state.as<SolveState>());
     }
 
-    bool column_solves(int precond) const {
-        return is3d && (precond == CISMGPU_PRECOND_SIA || precond == CISMGPU_PRECOND_TRIDIAG_LOCAL ||
-                        precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL);
-    }
+    bool column_solves(int precond) const { return is3d && (precond == CISMGPU_PRECOND_SIA || tri_precond(precond)); }
 
     // What a preconditioner needs of the matrix, once per solve (after k_init_state: a zero pivot
     // of the line preconditioners ends the solve with EDIVZERO).
     int precond_setup(int precond) {
-        if (precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL) {
+        if (tri_precond(precond)) {
             TRY(tri_setup(precond));
             // the line solution's planes: the lines write the same positions every time
             CU(cudaMemsetAsync(tri.as<double>() + TZS_U * g.NQ, 0, 2 * g.NQ * sizeof(double), stream));
         }
         if (column_solves(precond)) {
-            CU(sia.ensure((size_t)4 * nvec * sizeof(double)));
             k_sia_factor<<<dim3(nblocks(g.NQ, 128), 2), 128, 0, stream>>>(g, A.as<double>(), act.as<int32_t>(),
-                                                                          sia.as<double>());
+                                                                          column_pivots());
             CU(cudaGetLastError());
         }
         return CISMGPU_OK;
@@ -1195,7 +1198,7 @@ struct Solver {
     int precond_step(int upd, int precond, RedCtx rc, int setd = 0) {
         const Ptrs p = ptrs();
         SolveState *st = state.as<SolveState>();
-        const bool tri_pc = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
+        const bool tri_pc = tri_precond(precond);
         const long long bs = (long long)NCC * nvec, cd = (long long)(NCC / 2) * nvec;
         const double *Au = A.as<double>(), *Av = Au + 3 * bs;
         ColArgs c{};
@@ -1223,7 +1226,7 @@ struct Solver {
         }
         c.upd = upd;
         if (column_solves(precond)) {
-            c.fac = sia.as<double>();
+            c.fac = column_pivots();
             c.lo[0] = Au + 4 * nvec;
             c.lo[1] = Av + 4 * nvec;
             if (g.nz <= 16) col<P_SIA, DOT, 16>(c, rc);
@@ -1331,9 +1334,9 @@ int Solver::run_standard(int precond, int ncheck, double tol, int maxiters) {
     const Geom gg = g;
     prof_bytes = mv_bytes(0);
 
-    TRY(matrix_setup(maxiters));
+    TRY(matrix_setup(precond, maxiters));
     const MvMatrix M = matrix();
-    double *T = terms.as<double>();
+    double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
     halo(p.xu, p.xv);
@@ -1383,9 +1386,9 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     const bool tri = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
     if (tri && NCC == 9) maxiters = 100;
 
-    TRY(matrix_setup(maxiters));
+    TRY(matrix_setup(precond, maxiters));
     const MvMatrix M = matrix();
-    double *T = terms.as<double>();
+    double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     // r = d = z = q = Az = 0 (:3048-3061)
@@ -1442,9 +1445,9 @@ int Solver::run_standard_repro(int precond, int ncheck, double tol, int maxiters
     const Geom gg = g;
     double S0 = 0.0;
 
-    TRY(matrix_setup(maxiters));
+    TRY(matrix_setup(precond, maxiters));
     const MvMatrix M = matrix();
-    double *T = terms.as<double>();
+    double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
     halo(p.xu, p.xv);
@@ -1496,9 +1499,9 @@ int Solver::run_chrongear_repro(int precond, int ncheck, double tol, int maxiter
     if (tri && NCC == 9) maxiters = 100;
     double S0 = 0.0, S1 = 0.0;
 
-    TRY(matrix_setup(maxiters));
+    TRY(matrix_setup(precond, maxiters));
     const MvMatrix M = matrix();
-    double *T = terms.as<double>();
+    double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     CU(cudaMemsetAsync(p.ru, 0, (size_t)(VAZ_V - VR_U + 1) * nvec * sizeof(double), s));
@@ -1559,9 +1562,9 @@ int Solver::run_standard_seq(int precond, int ncheck, double tol, int maxiters) 
     const Geom gg = g;
     prof_bytes = mv_bytes(0);
 
-    TRY(matrix_setup(maxiters));
+    TRY(matrix_setup(precond, maxiters));
     const MvMatrix M = matrix();
-    double *T = terms.as<double>();
+    double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:1083-1160 / :263-376)
     halo(p.xu, p.xv);
@@ -1609,9 +1612,9 @@ int Solver::run_chrongear_seq(int precond, int ncheck, double tol, int maxiters)
     const bool tri = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
     if (tri && NCC == 9) maxiters = 100;
 
-    TRY(matrix_setup(maxiters));
+    TRY(matrix_setup(precond, maxiters));
     const MvMatrix M = matrix();
-    double *T = terms.as<double>();
+    double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
     TRY(precond_setup(precond));  // pcg_precond_init (:2916-3040 / :1747-1880)
     CU(cudaMemsetAsync(p.ru, 0, (size_t)(VAZ_V - VR_U + 1) * nvec * sizeof(double), s));
@@ -3756,8 +3759,7 @@ int cismgpu_solver_profile_read(cismgpu_solver_t *h, double *total_ms, int *laun
 size_t cismgpu_solver_device_bytes(const cismgpu_solver_t *h) {
     if (!h) return 0;
     const Solver &s = h->sv;
-    return s.A.n + s.raw.n + s.vec.n + s.act.n + s.partials.n + s.state.n + s.map.n + s.half.n + s.terms.n +
-           s.sia.n + s.mixed.bytes();
+    return s.A.n + s.raw.n + s.vec.n + s.act.n + s.partials.n + s.state.n + s.map.n + s.half.n + s.mixed.bytes();
 }
 
 int cismgpu_solver_destroy(cismgpu_solver_t *h) {

@@ -63,3 +63,20 @@ def test_matrix_changes_on_a_handle(gpu_lib, alg):
         assert got[0] == want[0]
         assert np.array_equal(got[1][0], want[1][0]) and np.array_equal(got[1][1], want[1][1])
     s.close()
+
+
+@pytest.mark.parametrize("precond", [1, 2, 3, 4])
+@pytest.mark.parametrize("reprosum", [0, 1])
+def test_fp64_solve_takes_no_vectors_of_its_own(gpu_lib, precond, reprosum):
+    """Below the half's size, a 3D solve's dot terms and column pivots add nothing to the handle (its bytes leave out the
+    line preconditioners' planes and reprosum's product fields): where the handle fitted, so does its solve."""
+    import cism_b200 as cg
+    P = asm.ice_stream(40, 37, NZ, seed=3)
+    P.par = dict(P.par, reprosum=reprosum)
+    s = cg.DeviceSolver(P)
+    before = s.device_bytes()
+    s.solve(cg.ALG_CHRONGEAR, precond, 5, 1e-30, 10)
+    s.solve(cg.ALG_STANDARD, precond, 5, 1e-30, 10)
+    grown = s.device_bytes() - before
+    s.close()
+    assert grown == 0
