@@ -1044,8 +1044,10 @@ struct Solver {
     }
 
     double mv_bytes(int extra_vec_streams) const {
-        // per active owned node: 4 blocks x NC coefficients + vector streams of 2 components
-        return (double)n_active_owned * g.nz * (4.0 * NC * 8.0 + 2.0 * 8.0 * (2 + extra_vec_streams));
+        // per active owned node: 4 blocks x the couplings read from HBM (NC, or the half's 14) + vector
+        // streams of 2 components; after matrix_setup
+        const double couplings = matrix().layout == MV_HALF ? 14.0 : NC;
+        return (double)n_active_owned * g.nz * (4.0 * couplings * 8.0 + 2.0 * 8.0 * (2 + extra_vec_streams));
     }
 
     // Device planes of the line-system couplings for precond 3/4 (TriMap): the raw index m that
@@ -1332,9 +1334,9 @@ int Solver::run_standard(int precond, int ncheck, double tol, int maxiters) {
     const unsigned nb = nblocks(g.NQ);
     auto rc = [&](int epi, int iter) { return RedCtx{part, st, epi, iter}; };
     const Geom gg = g;
-    prof_bytes = mv_bytes(0);
 
     TRY(matrix_setup(precond, maxiters));
+    prof_bytes = mv_bytes(0);
     const MvMatrix M = matrix();
     double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
@@ -1381,12 +1383,12 @@ int Solver::run_chrongear(int precond, int ncheck, double tol, int maxiters) {
     const unsigned nb = nblocks(g.NQ);
     auto rc = [&](int epi, int iter) { return RedCtx{part, st, epi, iter}; };
     const Geom gg = g;
-    prof_bytes = mv_bytes(1);  // the fused (r,z) dot also reads r
     // 2D with a tridiagonal preconditioner: at most 100 iterations (:1704-1732); 3D keeps maxiters
     const bool tri = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
     if (tri && NCC == 9) maxiters = 100;
 
     TRY(matrix_setup(precond, maxiters));
+    prof_bytes = mv_bytes(1);  // the fused (r,z) dot also reads r
     const MvMatrix M = matrix();
     double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
@@ -1560,9 +1562,9 @@ int Solver::run_standard_seq(int precond, int ncheck, double tol, int maxiters) 
     const int32_t *ac = act.as<int32_t>();
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
-    prof_bytes = mv_bytes(0);
 
     TRY(matrix_setup(precond, maxiters));
+    prof_bytes = mv_bytes(0);
     const MvMatrix M = matrix();
     double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);
@@ -1608,11 +1610,11 @@ int Solver::run_chrongear_seq(int precond, int ncheck, double tol, int maxiters)
     const int32_t *ac = act.as<int32_t>();
     const RedCtx none{part, st, EPI_NONE, 0};
     const Geom gg = g;
-    prof_bytes = mv_bytes(1);
     const bool tri = precond == CISMGPU_PRECOND_TRIDIAG_LOCAL || precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
     if (tri && NCC == 9) maxiters = 100;
 
     TRY(matrix_setup(precond, maxiters));
+    prof_bytes = mv_bytes(1);
     const MvMatrix M = matrix();
     double *T = dot_terms();
     k_init_state<<<1, 1, 0, s>>>(st, tol, maxiters);

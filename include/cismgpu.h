@@ -619,7 +619,8 @@ int cismgpu_solver_assemble_stiffness_2d(cismgpu_solver_t *s, int nz, int nhalo,
 
 /* Per-kernel CUDA-event timing of the structured matvec launches (off by default).
  * read: total device milliseconds, launch count, and algorithmic bytes per launch
- * (active owned nodes x (4*NC*sizeof(A) + vector streams)). */
+ * (active owned nodes x (4*couplings*sizeof(A) + vector streams); couplings: NC, or 14
+ * where the matvecs read the symmetric half of a 3D matrix). */
 int cismgpu_solver_profile(cismgpu_solver_t *s, int enable);
 int cismgpu_solver_profile_read(cismgpu_solver_t *s, double *total_ms, int *launches, double *bytes_per_launch);
 

@@ -80,3 +80,20 @@ def test_fp64_solve_takes_no_vectors_of_its_own(gpu_lib, precond, reprosum):
     grown = s.device_bytes() - before
     s.close()
     assert grown == 0
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_profiled_bytes_of_a_product(gpu_lib, symmetric):
+    """The half's 14 couplings, or all 27: x and y, and r for the fused dot products."""
+    import cism_b200 as cg
+    P = matrix(symmetric)
+    p = P.par
+    own = P.active_vertex[p["staggered_jlo"] - 1:p["staggered_jhi"], p["staggered_ilo"] - 1:p["staggered_ihi"]]
+    n = np.count_nonzero(own) * NZ
+    s = cg.DeviceSolver(P)
+    s.profile()
+    s.solve(cg.ALG_CHRONGEAR, 2, 5, 1e-30, 10)
+    _, launches, nbytes = s.profile_read()
+    s.close()
+    assert launches == 9
+    assert nbytes == n * (4 * (14 if symmetric else 27) * 8 + 3 * 16)
