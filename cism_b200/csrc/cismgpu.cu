@@ -2192,15 +2192,21 @@ static std::string tile_key_batch(bool is3d, int nzm) {
     return std::string("batch:") + (is3d ? "3d" : "2d") + ":nzm" + std::to_string(nzm);
 }
 
+// Without a preconditioner the iteration count follows the rounding, and so the tiling: an 11 x 10 SSA system
+// takes 310 iterations at the rule's height, 265 to 430 at most others, 1295 at 6 and does not
+// converge in 5000 from 9 on, while their steps differ by a few percent.  Such solves keep the rule.
+static bool tiles_tuned(int precond) { return precond != CISMGPU_PRECOND_NONE; }
+
 // The single-solve tile height of sv (prepared with the default height, so its layout is set).
 static int tuned_solve_ty(Solver &sv, int precond, int nzm, int TYdef, int *TY) {
+    *TY = TYdef;
+    if (!tiles_tuned(precond)) return CISMGPU_OK;
     const std::string key = tile_key_single(sv, nzm);
     int v = g_tiles.get(key);
     if (v > 0 && mixed_grid(sv.is3d, nzm, v, false) > 0) {
         *TY = v;
         return CISMGPU_OK;
     }
-    *TY = TYdef;
     if (!g_tiles.timing_on()) return CISMGPU_OK;
     std::vector<int> cand = {TYdef};
     for (int ty : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32})
@@ -2226,8 +2232,8 @@ static int tuned_solve_ty(Solver &sv, int precond, int nzm, int TYdef, int *TY) 
     return CISMGPU_OK;
 }
 
-static int batch_floor(bool is3d, int nzm) {
-    const int v = g_tiles.get(tile_key_batch(is3d, nzm));
+static int batch_floor(bool is3d, int nzm, int precond) {
+    const int v = tiles_tuned(precond) ? g_tiles.get(tile_key_batch(is3d, nzm)) : 0;
     return v > 0 ? v : (is3d ? 4 : 16);
 }
 
@@ -2625,7 +2631,7 @@ static int batch_prepare(MixedBatch &B, int precond, int ncheck, double tol, int
     Solver &s0 = *B.svs[0];
     B.is3d = s0.is3d;
     B.nzm = mixed_nzm(s0.g, s0.is3d);
-    if (floor <= 0) floor = batch_floor(B.is3d, B.nzm);
+    if (floor <= 0) floor = batch_floor(B.is3d, B.nzm, precond);
     std::vector<int> tys(n);
     std::vector<MTile> tl;
     for (int t = 0; t < n; ++t) {
@@ -2715,7 +2721,7 @@ static int tune_batch_floor(const std::vector<Solver *> &svs, int precond, int n
     for (Solver *sv : svs)
         if (sv->is3d != is3d || mixed_nzm(sv->g, sv->is3d) != nzm) return CISMGPU_OK;  // batch_prepare rejects it
     const std::string key = tile_key_batch(is3d, nzm);
-    if (g_tiles.get(key) > 0 || !g_tiles.timing_on()) return CISMGPU_OK;
+    if (!tiles_tuned(precond) || g_tiles.get(key) > 0 || !g_tiles.timing_on()) return CISMGPU_OK;
     const int fdef = is3d ? 4 : 16;
     const std::vector<int> cand = is3d ? std::vector<int>{4, 2, 6, 8} : std::vector<int>{16, 8, 32};
     float tdef = 0.f, tbest = 0.f;

@@ -129,7 +129,7 @@ static int srv_admit(SrvReq &r) {
     r.h = h;
     Solver &sv = h->sv;
     const int nzm = mixed_nzm(sv.g, sv.is3d);
-    r.TY = mixed_batch_ty(sv.g, sv.is3d, nzm, batch_floor(sv.is3d, nzm));
+    r.TY = mixed_batch_ty(sv.g, sv.is3d, nzm, batch_floor(sv.is3d, nzm, q.precond));
     if (!sv.is3d) {
         // a large 2D system runs its epochs on the single-solve kernel, a launch of its own, with
         // its FP32 matrix resident in shared memory where the tiles fit one per co-resident CTA
