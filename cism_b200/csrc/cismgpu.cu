@@ -1211,18 +1211,19 @@ struct Solver {
             else if (upd == U_XR) node<U_XR>();
             if (upd != U_RHALO) upd = U_NONE;
             const int global = precond == CISMGPU_PRECOND_TRIDIAG_GLOBAL;
-            const int pending = upd == U_RHALO;  // the halo of r follows the lines, which read it as updated
+            // the halo of r follows the lines, which read r as it will leave it
+            const bool pending = upd == U_RHALO && halo_reaches_owned(g);
             double *T = tri.as<double>();
             const long long NQ = g.NQ;
             if (NCC == 27) {
-                launch_dep(k_tri_lines<true>, dim3(tri_blocks(g)), kTriThreads, tri_smem(g), stream, g, global, pending,
-                           p.ru, p.rv, T + TZS_U * NQ, T + TZS_V * NQ, T, st);
+                launch_dep(pending ? k_tri_lines<true, true> : k_tri_lines<true, false>, dim3(tri_blocks(g)), kTriThreads,
+                           tri_smem(g), stream, g, global, p.ru, p.rv, T + TZS_U * NQ, T + TZS_V * NQ, T, st);
                 c.zs = T + TZS_U * NQ;
             } else {
                 CU(cudaMemsetAsync(p.zu, 0, NQ * sizeof(double), stream));
                 CU(cudaMemsetAsync(p.zv, 0, NQ * sizeof(double), stream));
-                launch_dep(k_tri_lines<false>, dim3(tri_blocks(g)), kTriThreads, tri_smem(g), stream, g, global, pending,
-                           p.ru, p.rv, p.zu, p.zv, T, st);
+                launch_dep(pending ? k_tri_lines<false, true> : k_tri_lines<false, false>, dim3(tri_blocks(g)), kTriThreads,
+                           tri_smem(g), stream, g, global, p.ru, p.rv, p.zu, p.zv, T, st);
                 halo(p.zu, p.zv);
             }
         }

@@ -435,6 +435,16 @@ __device__ __forceinline__ long long halo_src(const Geom &g, int i, int j, long 
     return q;
 }
 
+// The staggered halo update writes owned positions (no_ice: the last owned row and column in the
+// reference's geometry).
+inline bool halo_reaches_owned(const Geom &g) {
+    auto in = [&](int lo, int hi, int N) {
+        if (g.outflow ? (lo <= 0 || hi >= N - 1) : (g.no_ice && (lo <= 1 || hi >= N - 2))) return true;
+        return g.periodic && (lo <= 1 || hi >= N - 1);
+    };
+    return in(g.ilo, g.ihi, g.NX) || in(g.jlo, g.jhi, g.NY);
+}
+
 // a(i, j) = v followed by the staggered halo update of a, by the thread of (i, j) alone: a zero
 // position stores zero, a periodic halo position nothing, any other its value and its images.
 __device__ __forceinline__ void put_haloed(const Geom &g, int i, int j, double *__restrict__ a, double v) {
@@ -1166,8 +1176,9 @@ __global__ void k_tri_factor(Geom g, int global, double *__restrict__ T, SolveSt
 // Line solves of tridiag_solver_local_2d (:4985-5013 u, :5041-5069 v) from planes bu, bv into
 // xu, xv, which hold zeros outside the lines: gamma forward, then back substitution.  SUM (3D): the
 // right-hand side is the sum of r over the levels, in level order (tridiag_solver_local_3d :4585-4590).
-// pending: the halo update of b is still to come (U_RHALO, by the kernel that follows); it may reach
-// owned positions (no_ice zeroes the last owned row and column), so the lines read what it will leave.
+// PENDING: the halo update of b is still to come (U_RHALO, by the kernel that follows) and reaches owned
+// positions (halo_reaches_owned), so the lines read what it will leave.  A variant of its own: the test
+// in every staged element cost a 150x101x11 solve 6 % where no update reaches an owned position.
 // A line is a chain of dependent FP64 operations (three a position forward, two backward), which
 // bounds the launch; so everything else is taken off the chain: a block stages kTriLines lines,
 // kTriChunk positions at a time, in shared memory with all its threads (coalesced for the u lines,
@@ -1178,8 +1189,8 @@ __global__ void k_tri_factor(Geom g, int global, double *__restrict__ T, SolveSt
 constexpr int kTriLines = 4, kTriChunk = 376, kTriThreads = 128;
 static_assert(4 * kTriLines * (kTriChunk + 1) * sizeof(double) <= 48 * 1024, "no opt-in shared memory");
 
-template <bool SUM>
-__global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, int pending, const double *__restrict__ bu,
+template <bool SUM, bool PENDING>
+__global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, const double *__restrict__ bu,
                                                            const double *__restrict__ bv, double *__restrict__ xu,
                                                            double *__restrict__ xv, const double *__restrict__ T,
                                                            const SolveState *st) {
@@ -1210,12 +1221,12 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, i
         const int c0 = c * kTriChunk, n = min(kTriChunk, len - c0);
         each(c0, n, [&](int w, long long e) {
             long long f = e;
-            if (pending) {
+            if (PENDING) {
                 const int j = (int)e / g.NX, i = (int)e - j * g.NX;
                 f = halo_src(g, i, j, e);
             }
             double v = 0.0;
-            if (SUM && f >= 0) {
+            if (SUM && (!PENDING || f >= 0)) {
                 for (int k0 = 0; k0 < g.nz; k0 += 8) {
                     double r[8];
 #pragma unroll
@@ -1224,7 +1235,7 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_lines(Geom g, int global, i
                     for (int u = 0; u < 8; ++u)
                         if (k0 + u < g.nz) v = __dadd_rn(v, r[u]);
                 }
-            } else if (f >= 0) {
+            } else if (!PENDING || f >= 0) {
                 v = b[f];
             }
             sb[w] = v;

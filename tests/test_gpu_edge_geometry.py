@@ -29,7 +29,8 @@ def system(dims, edges, bc="none", seed=1):
     A[3, ..., nc // 2] += 12.0
     b = rng.standard_normal((2, NY, NX, nz))
     active = (rng.random((NY, NX)) > 0.1).astype(np.int32)
-    par = dict(asm.default_par(nx, ny, bc="outflow"), periodic_bc=0, outflow_bc=0, no_ice_bc=int(bc == "no_ice"))
+    par = dict(asm.default_par(nx, ny, bc="outflow"), periodic_bc=int(bc == "periodic"),
+               outflow_bc=int(bc == "outflow"), no_ice_bc=int(bc == "no_ice"))
     par.update({"ilo": dict(staggered_ilo=1), "ihi": dict(staggered_ihi=nx - 1), "jlo": dict(staggered_jlo=1),
                 "jhi": dict(staggered_jhi=ny - 1), "all": dict(staggered_ilo=1, staggered_ihi=nx - 1, staggered_jlo=1,
                                                                staggered_jhi=ny - 1)}[edges])
@@ -51,8 +52,8 @@ def test_systems_are_solvable():
 @pytest.mark.gpu
 @pytest.mark.parametrize("alg", ["standard", "chrongear"])
 @pytest.mark.parametrize("dims,precond", [(d, p) for d in (2, 3) for p in range(5) if (d, p) != (2, 2)])
-@pytest.mark.parametrize("edges,bc", [("all", "none"), ("all", "no_ice"), ("ilo", "none"), ("ihi", "none"), ("jlo", "none"),
-                                      ("jhi", "none")])
+@pytest.mark.parametrize("edges,bc", [("all", "none"), ("all", "no_ice"), ("all", "outflow"), ("jlo", "outflow"),
+                                      ("ilo", "none"), ("ihi", "none"), ("jlo", "none"), ("jhi", "none")])
 def test_fp64_solve(gpu_lib, dims, edges, bc, precond, alg):
     import cism_b200 as cg
     P = system(dims, edges, bc)
