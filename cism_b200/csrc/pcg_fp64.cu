@@ -1075,36 +1075,30 @@ __global__ void k_tri_coef(Geom g, const double *__restrict__ A, const int32_t *
     const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
     if (q >= g.NQ) return;
     const long long plane = (long long)g.nz * g.NQ;
+    // 3D, global: the staggered halo update of the nine summed planes (:4055-4058) is taken on the way: the
+    // column s whose sums q holds after it, or zero.  With no_ice it reaches the last owned row and
+    // column, otherwise owned positions only where these lie in the halo.
+    const long long s = (NC == 27 && global) ? halo_src(g, (int)(q % g.NX), (int)(q / g.NX), q) : q;
     for (int comp = 0; comp < 2; ++comp) {
         const double *B = A + (comp ? 3LL : 0LL) * NC * plane;  // Auu or Avv
-        double v[3];
-        for (int e = 0; e < 3; ++e) {
+        double v[3] = {0.0, 0.0, 0.0};
+        for (int e = 0; e < 3 && s >= 0; ++e) {
             if (NC == 9) {
                 v[e] = B[(long long)tm.c[comp][e][0] * g.NQ + q];
             } else {
                 double sum = 0.0;
                 for (int k = 0; k < g.nz; ++k) {
-                    const long long o = (long long)k * g.NQ + q;
+                    const long long o = (long long)k * g.NQ + s;
                     sum = __dadd_rn(__dadd_rn(__dadd_rn(sum, B[tm.c[comp][e][0] * plane + o]),
                                               B[tm.c[comp][e][1] * plane + o]),
                                     B[tm.c[comp][e][2] * plane + o]);
                 }
-                if (act[q] == 0) {
+                if (act[s] == 0) {
                     if (tm.m[comp][e] == 5) sum = 1.0;
                     else if (!global) sum = 0.0;
                 }
                 v[e] = sum;
             }
-        }
-        if (NC == 27 && global) {
-            // the global form's staggered halo update of the nine summed planes (:4055-4058): its
-            // outflow / no_ice zeroing, which with no_ice reaches the last owned row and column
-            // (its periodic copies reach only halo positions, which no owned line reads)
-            const int i = (int)(q % g.NX), j = (int)(q / g.NX);
-            bool zero = false;
-            if (g.outflow) zero = (i == 0 || i == g.NX - 1 || j == 0 || j == g.NY - 1);
-            else if (g.no_ice) zero = (i <= 1 || i >= g.NX - 2 || j <= 1 || j >= g.NY - 2);
-            if (zero) v[0] = v[1] = v[2] = 0.0;
         }
         if (v[1] == 0.0) { v[1] = 1.0; v[0] = 0.0; v[2] = 0.0; }
         double *P = T + (comp ? TV_SUB : TU_SUB) * g.NQ;

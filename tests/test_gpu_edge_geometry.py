@@ -53,7 +53,8 @@ def test_systems_are_solvable():
 @pytest.mark.parametrize("alg", ["standard", "chrongear"])
 @pytest.mark.parametrize("dims,precond", [(d, p) for d in (2, 3) for p in range(5) if (d, p) != (2, 2)])
 @pytest.mark.parametrize("edges,bc", [("all", "none"), ("all", "no_ice"), ("all", "outflow"), ("jlo", "outflow"),
-                                      ("ilo", "none"), ("ihi", "none"), ("jlo", "none"), ("jhi", "none")])
+                                      ("all", "periodic"), ("ihi", "periodic"), ("ilo", "none"), ("ihi", "none"),
+                                      ("jlo", "none"), ("jhi", "none")])
 def test_fp64_solve(gpu_lib, dims, edges, bc, precond, alg):
     import cism_b200 as cg
     P = system(dims, edges, bc)
