@@ -198,14 +198,14 @@ static int check_device() {
 }
 
 static inline unsigned nblocks(long long n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
-// An FP64 3D solve builds the symmetric half of its matrix from this size of the full blocks and this
-// many iterations on: below, L2 keeps the planes and both products take 6.3 us (40x40x11 to 64x64x11;
-// 96x96x11 10.4 us from the planes, 9.3 from the half; 149x100x11 26.8 and 14.5; 201x201x11 59.7 and
-// 37.0), and the copy costs what three products save.
+// An FP64 3D solve builds the symmetric half of its matrix from this size of the full blocks on, where its
+// caller allows this many iterations (maxiters: how many it will take is not known): below, L2 keeps the
+// planes and both products take 6.3 us (40x40x11 to 64x64x11; 96x96x11 10.4 us from the planes, 9.3 from
+// the half; 149x100x11 26.8 and 14.5; 201x201x11 59.7 and 37.0), and the copy costs what three products save.
 constexpr size_t kHalfMinBytes = 64u << 20;
 constexpr int kHalfMinIters = 8;
-// rows of blocks (planes in parallel) for the halo of a matrix's 27 nz coefficient planes: with 64 rows each
-// went through 5 planes of an 11-level matrix one after the other, 12.4 us a pair of blocks; now 7.6.
+// rows of blocks (planes in parallel) for the halo of a matrix's 27 nz coefficient planes: 7.6 us a pair of blocks
+// at 201x161x11; with 64 rows, five planes one after the other, 12.4.
 constexpr unsigned kHaloPlaneRows = 512;
 static inline bool is_check(int iter, int ncheck) { return (iter % ncheck == 0) || iter == 5; }
 

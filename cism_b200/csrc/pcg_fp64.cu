@@ -300,8 +300,9 @@ constexpr int kDotChunk = 8;  // levels whose loads a column's dot terms issue t
 // sums of the early column blocks overlapping the rest of the matvec.  The per-column-block
 // counters sit after the partials and return to zero here.  In 2D a column has one level, so
 // every block reduces its own terms.
-// 2D: five blocks an SM, so that the 638 blocks of a 401x401 grid run at once (three: 99 ms a solve
-// against 87).
+// 2D: five blocks an SM (48 registers).  Microseconds an iteration with 3, 4, 5 and 6: 201x201 16.4, 16.1,
+// 17.5, 18.0; 301x301 19.3, 20.0, 19.2, 20.8; 401x401 25.7, 25.8, 23.0, 23.5; 601x601 56.4, 53.8, 50.2, 52.0;
+// 801x801 90.2, 86.4, 85.2, 85.1; equal up to 121x121.
 template <int NC, int MODE, int LAY>
 __global__ void __launch_bounds__(kBlock, NC == 9 ? 5 : 3) k_mv_nodes(Geom g, MvMatrix M, const int32_t *__restrict__ act,
                                                         const double *__restrict__ xu, const double *__restrict__ xv,
@@ -406,8 +407,9 @@ inline void launch_mv(cudaStream_t s, const Geom &g, const MvMatrix &M, const in
 // taken at the same time: a halo position reads its source (halo_src), or the source's thread
 // writes its images (put_haloed).  Both give the values the reference's separate update leaves.
 // With one launch per statement group and one thread per column walking its levels, an iteration
-// of the 201x201x11 ice stream spent 90 us of 190 here, and its solve took 5.42 ms against 3.88 ms
-// now (SIA); the 31x31x11 dome 2.16 against 1.08 ms, SSA 401x401 (diagonal) 161 against 113 ms.
+// of the 201x201x11 ice stream spent 90 us of 190 here.  Joining them took its solve from 5.42 to 3.88 ms
+// (SIA), the 31x31x11 dome from 2.16 to 1.08 and SSA 401x401 (diagonal) from 161 to 113; with the half,
+// the dependent launches and the 2D product's blocks these are 2.58, 0.78 and 84 ms.
 
 // Positions of the staggered halo that hold zero (outflow, no_ice).
 __device__ __forceinline__ bool zero_pos(const Geom &g, int i, int j) {
@@ -1173,8 +1175,8 @@ __global__ void k_tri_factor(Geom g, int global, double *__restrict__ T, SolveSt
 // PENDING: the halo update of b is still to come (U_RHALO, by the kernel that follows) and reaches owned
 // positions (halo_reaches_owned), so the lines read what it will leave.  A variant of its own: the test
 // in every staged element cost a 150x101x11 solve 6 % where no update reaches an owned position.
-// A line is a chain of dependent FP64 operations (three a position forward, two backward), which
-// bounds the launch; so everything else is taken off the chain: a block stages kTriLines lines,
+// A line is a chain of dependent FP64 operations (three a position forward, two backward; 66 ns a
+// position, 10 of the 22 us below), so everything else is taken off the chain: a block stages kTriLines lines,
 // kTriChunk positions at a time, in shared memory with all its threads (coalesced for the u lines,
 // whole 32-byte sectors for the v lines, kTriLines adjacent columns), one thread per line runs the
 // recurrences there, and all threads store.  The operations and their order are the reference's.

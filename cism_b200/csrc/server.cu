@@ -336,9 +336,9 @@ static void srv_admit_loop(cismgpu_server *S) {
 // join at the next epoch.  The host waits for each epoch before it queues the next: a pipelined
 // form that queued epoch e before reading e-1 measured slower on the served stream (6.9 against
 // 8.3 solves/s), because a 3D result's layout change is a kernel that cannot start beside a
-// cooperative launch holding every SM, and freeing a finished request's memory synchronizes the
-// device, so the host waited for the queued epoch anyway and every request spent one more epoch
-// as a skipped member.
+// cooperative launch holding every SM, and every request spent one more epoch as a skipped member.
+// (Freeing a finished request's memory also synchronized the device then; its blocks are kept now,
+// so that part of the measurement no longer holds.)
 static void srv_loop(cismgpu_server *S) {
     cudaSetDevice(S->device);
     SrvLaunch L[kSrvClasses];

@@ -1,7 +1,7 @@
 """Chronopoulos-Gear with the line preconditioners where the staggered halo update of r reaches owned
 vertices: under no_ice it zeroes the last owned row and column, which the lines run through, and the
-reference updates r before its first preconditioner and after every check (glissade_velo_higher_pcg.F90
-:3118-3121, :3518-3520).  The systems were not halo-updated by their caller, so r = b - A x is not zero
+reference updates r before its first preconditioner (glissade_velo_higher_pcg.F90:3118-3121) and after
+every check.  The systems were not halo-updated by their caller, so r = b - A x is not zero
 there beforehand.  Bit for bit against the oracle, in every order of the global sums."""
 import contextlib
 
