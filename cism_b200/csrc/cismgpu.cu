@@ -2692,6 +2692,7 @@ static int batch_prepare(MixedBatch &B, int precond, int ncheck, double tol, int
     CU(cudaMemcpy(B.d_tiles, tl.data(), tl.size() * sizeof(MTile), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(B.d_dst, dst.data(), n * sizeof(SolveState *), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(B.d_ctl0, &c0, sizeof(MCtl), cudaMemcpyHostToDevice));
+    CU(cudaStreamSynchronize(cudaStreamLegacy));  // a pageable copy may return before its DMA, and non-blocking streams do not wait for it
     return CISMGPU_OK;
 }
 
